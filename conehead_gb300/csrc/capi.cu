@@ -719,6 +719,22 @@ BeamDev make_beam(const ch_beam& in, const ch_grid& g, int samples) {
   b.full_rows = in.full_rows;
   b.full_cols = in.full_cols;
   b.uniform = in.block_uniform;
+  // sub-sample lattice: samples lie within s (S - 1) / (2 S) of the centre per axis
+  b.lat = in.geom_f32 ? 0 : 1;
+  b.wraps = (r1 == in.full_rows - 1 || c1 == in.full_cols - 1) ? 1 : 0;
+  for (int k = 0; k < 3; ++k) {
+    const float h = 1.0001f * g.spacing[k] * (float)(samples - 1) / (2.0f * samples);
+    b.lat_n += h * std::fabs(b.vyf[k]);
+    b.lat_0 += h * std::fabs(b.m0f[k]);
+    b.lat_2 += h * std::fabs(b.m2f[k]);
+  }
+  // map index r is read by cell r - 1999, cells -1999..1999 (the wrapped one aside)
+  b.rlim = std::max(0, std::min(in.block_rows, 3999 - in.block_r0));
+  b.clim = std::max(0, std::min(in.block_cols, 3999 - in.block_c0));
+  b.uc = (float)(in.block_r0 - 1999) + 0.5f * (float)b.rlim;
+  b.uh = 0.5f * (float)b.rlim;
+  b.wc = (float)(in.block_c0 - 1999) + 0.5f * (float)b.clim;
+  b.wh = 0.5f * (float)b.clim;
   b.sad = in.sad;
   b.sad_f32 = in.sad_f32;
   return b;

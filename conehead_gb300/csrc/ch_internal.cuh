@@ -104,6 +104,12 @@ struct BeamDev {
   const float* block;
   int brows, bcols, br0, bc0, full_rows, full_cols;
   int uniform;          // every crop value is 1.0
+  // sub-sample lattice (blocked_fraction)
+  int lat;              // float64 source arrays: samples may be classified in float32
+  int wraps;            // the crop holds the map's last row or column, which index -2000 reads
+  float lat_n, lat_0, lat_2;   // largest |d nd|, |d x0|, |d x2| of a sub-sample from its voxel centre (cm)
+  float uc, uh, wc, wh; // the crop's cells, centre and half width along u (rows) and w (columns)
+  int rlim, clim;       // crop rows and columns a lookup can reach without the wrap
   // fluence / TERMA
   double sad;
   int sad_f32;

@@ -29,6 +29,8 @@ constexpr float SAMPLE_DELTA = 0.05f;   // cells (0.1 mm) of float32 slack
 // partial sums 0, 1/27, 1/27+1/27, ... accumulated in float64 as the
 // reference does for a block value of exactly 1.0 and 3x3x3 samples
 __constant__ double c_unit_partial[28];
+// the same sums over all S^3 sub-samples, S = 1..16
+__constant__ double c_unit_sum[17];
 
 // --------------------------------------------------------- block lookup --
 // cell index i = floor(100 x) (x in cm, beam coordinates); the reference
@@ -197,145 +199,148 @@ __device__ __noinline__ double blocked_general(const BeamDev& b, const GridDev& 
   return acc;
 }
 
-// Blocked fraction of one voxel where it is decided without classifying the
-// 3x3x3 samples one by one (returns false when they are needed): the general
-// sum (other sample counts, float32 source arrays), and for a uniform jaw
-// crop a voxel wholly inside or wholly outside the opening.
-__device__ __forceinline__ bool blocked_quick(const BeamDev& b, const GridDev& g, int S, const float* pos, int& bad,
-                                              double& out) {
-  if (S != 3 || b.geom_f32) {
-    out = blocked_general(b, g, S, pos, bad);
-    return true;
-  }
-  float off[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) off[k] = fdiv(g.spacing[k], 3.0f);
-  if (b.uniform) {
-    // Fast test for a voxel wholly inside a jaw opening.  The samples lie in
-    // the box of the extreme ones (offsets -s/3 and +s/3 per axis).  On the
-    // source's side of the plane the projection through the source maps
-    // segments to segments, so every sample's cell lies in the cell box of
-    // the 8 corner projections, widened by the same float32 error bound as a
-    // single sample.  The open cells of a uniform crop form a rectangle (the
-    // -1 wrap at index -2000 excluded), so when both extreme cells of the box
-    // are open every sample is open: blocked is the reference's sum of 27
-    // ones.  Otherwise the samples are classified one by one.
-    float umin = 3.0e38f, umax = -3.0e38f, wmin = 3.0e38f, wmax = -3.0e38f;
-    bool ok = true;
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const float rx = off[0] * ((c & 1) ? 2.5f : 0.5f) - g.spacing[0] * 0.5f;
-      const float ry = off[1] * ((c & 2) ? 2.5f : 0.5f) - g.spacing[1] * 0.5f;
-      const float rz = off[2] * ((c & 4) ? 2.5f : 0.5f) - g.spacing[2] * 0.5f;
-      const float p0 = pos[0] + rx, p1 = pos[1] + ry, p2 = pos[2] + rz;
-      const float np_ = b.vyf[0] * p0 + b.vyf[1] * p1 + b.vyf[2] * p2;
-      const float m0p = b.m0f[0] * p0 + b.m0f[1] * p1 + b.m0f[2] * p2;
-      const float m2p = b.m2f[0] * p0 + b.m2f[1] * p1 + b.m2f[2] * p2;
-      const float ndr = b.a_nS - np_;
-      ok = ok && fabsf(ndr) > 0.2f * fabsf(b.a_K);
-      const float si = __fdividef(b.a_K, ndr);
-      const float ux = (b.a_c0 + si * (b.a_m0S - m0p)) * 100.0f;
-      const float uz = (b.a_c2 + si * (b.a_m2S - m2p)) * 100.0f;
-      umin = fminf(umin, ux);
-      umax = fmaxf(umax, ux);
-      wmin = fminf(wmin, uz);
-      wmax = fmaxf(wmax, uz);
-    }
-    if (ok) {
-      const int i0 = floor_cell(umin - SAMPLE_DELTA), i1 = floor_cell(umax + SAMPLE_DELTA);
-      const int k0 = floor_cell(wmin - SAMPLE_DELTA), k1 = floor_cell(wmax + SAMPLE_DELTA);
-      if (i0 > -2000 && k0 > -2000) {
-        if (cell_value(b, i0, k0) == 1.0f && cell_value(b, i1, k1) == 1.0f) {
-          out = c_unit_partial[27];
-          return true;
-        }
-        // Wholly closed: the box misses the open rectangle of cells
-        // i in [br0 - 1999, br0 + brows - 2000], k likewise (within the map's
-        // [-1999, 1999]; the wrapped index -2000 is outside the box), so
-        // every sample reads 0 and blocked is the reference's sum of zeros.
-        const int oi0 = max(b.br0 - 1999, -1999), oi1 = min(b.br0 + b.brows - 2000, 1999);
-        const int ok0 = max(b.bc0 - 1999, -1999), ok1 = min(b.bc0 + b.bcols - 2000, 1999);
-        if (i1 < oi0 || i0 > oi1 || k1 < ok0 || k0 > ok1) {
-          out = c_unit_partial[0];
-          return true;
-        }
+// -------------------------------------------------- sub-sample lattice --
+// The S^3 sub-samples are a lattice, so the three linear forms of the float32
+// projection -- nd = n.(S - p), x0 = m0.(S - p), x2 = m2.(S - p) -- step by
+// constants from sample to sample: a sample costs three FMAs, one fast
+// reciprocal and two FMAs for its cell coordinates
+//   u = 100 (c0 + K x0 / nd),   w = 100 (c2 + K x2 / nd),
+// where the per-sample dot products cost about thirty instructions.
+struct Centre {
+  float nd, x0, x2;     // the linear forms at the voxel centre
+  float u, w, mu, mw;   // its cell coordinates, and how far a sub-sample's may be from them
+};
+
+// Projects the voxel centre and bounds the sub-samples around it.  For an
+// offset of the lattice's box, |d nd| <= A = lat_n, |d x0| <= B = lat_0, so
+//   |d(K x0 / nd)| <= |K| (B + |x0 / nd| A) / (|nd| - A).
+// False when a sub-sample may lie closer to the source plane than 0.2 |K|
+// (the float32 error bound SAMPLE_DELTA assumes a magnification below 5) or
+// may read the wrapped cell -2000 of a crop that holds the map's last row or
+// column: those voxels, and float32 source arrays, take blocked_general.
+__device__ __forceinline__ bool lattice_centre(const BeamDev& b, const float* pos, Centre& c) {
+  if (!b.lat) return false;
+  c.nd = b.a_nS - (b.vyf[0] * pos[0] + b.vyf[1] * pos[1] + b.vyf[2] * pos[2]);
+  c.x0 = b.a_m0S - (b.m0f[0] * pos[0] + b.m0f[1] * pos[1] + b.m0f[2] * pos[2]);
+  c.x2 = b.a_m2S - (b.m2f[0] * pos[0] + b.m2f[1] * pos[1] + b.m2f[2] * pos[2]);
+  const float near = fabsf(c.nd) - b.lat_n;
+  if (!(near > 0.2f * fabsf(b.a_K))) return false;
+  const float K = 100.0f * b.a_K;
+  const float inv = __fdividef(1.0f, c.nd), mag = __fdividef(fabsf(K), near);
+  c.u = K * inv * c.x0 + 100.0f * b.a_c0;
+  c.w = K * inv * c.x2 + 100.0f * b.a_c2;
+  c.mu = mag * (b.lat_0 + fabsf(c.x0 * inv) * b.lat_n) + SAMPLE_DELTA;
+  c.mw = mag * (b.lat_2 + fabsf(c.x2 * inv) * b.lat_n) + SAMPLE_DELTA;
+  return !b.wraps || (c.u - c.mu > -1999.0f && c.w - c.mw > -1999.0f);
+}
+
+// Calls f(ix, iy, iz, u, w) for every sub-sample in the reference's order.
+template <class F>
+__device__ __forceinline__ void for_samples(const BeamDev& b, const float* off, int S, const Centre& c, F f) {
+  const float K = 100.0f * b.a_K, c0 = 100.0f * b.a_c0, c2 = 100.0f * b.a_c2;
+  const float mid = 0.5f * (float)(S - 1);
+#pragma unroll 1
+  for (int ix = 0; ix < S; ++ix) {
+    const float rx = off[0] * ((float)ix - mid);
+    const float nx = c.nd - b.vyf[0] * rx, x0x = c.x0 - b.m0f[0] * rx, x2x = c.x2 - b.m2f[0] * rx;
+#pragma unroll 1
+    for (int iy = 0; iy < S; ++iy) {
+      const float ry = off[1] * ((float)iy - mid);
+      const float ny = nx - b.vyf[1] * ry, x0y = x0x - b.m0f[1] * ry, x2y = x2x - b.m2f[1] * ry;
+#pragma unroll 3
+      for (int iz = 0; iz < S; ++iz) {
+        const float rz = off[2] * ((float)iz - mid);
+        const float si = __fdividef(K, ny - b.vyf[2] * rz);
+        f(ix, iy, iz, si * (x0y - b.m0f[2] * rz) + c0, si * (x2y - b.m2f[2] * rz) + c2);
       }
     }
   }
-  return false;
 }
 
-// sample sidx = 9 ix + 3 iy + iz of the 3x3x3 set: its float32 offset from
-// the voxel centre
-__device__ __forceinline__ float sample_of(const BeamDev& b, const GridDev& g, const float* pos, const float* off,
-                                           int sidx, int& bad) {
-  const int ix = sidx / 9, iy = (sidx / 3) % 3, iz = sidx % 3;
-  const float rx = off[0] * ((float)ix + 0.5f) - g.spacing[0] * 0.5f;
-  const float ry = off[1] * ((float)iy + 0.5f) - g.spacing[1] * 0.5f;
-  const float rz = off[2] * ((float)iz + 0.5f) - g.spacing[2] * 0.5f;
-  return sample_value(b, g, pos, off, rx, ry, rz, ix, iy, iz, bad);
+// floor of a coordinate clamped to +-1e6, as an integer: adding 1.5 2^23
+// rounding down leaves it in the low mantissa bits
+__device__ __forceinline__ int floor_int(float v) {
+  const float m = __fadd_rd(fminf(fmaxf(v, -1.0e6f), 1.0e6f), 12582912.0f);
+  return __float_as_int(m) - 0x4b400000;
 }
 
-// blocked fraction of one voxel; the 3x3x3 jaw case (values 0 and 1 only)
-// counts open samples and sums through the precomputed float64 partial sums
-// (the reference's float64 sum of n ones and 27 - n zeros, in any order)
-__device__ double blocked_fraction(const BeamDev& b, const GridDev& g, int S, const float* pos, int& bad) {
-  double quick;
-  if (blocked_quick(b, g, S, pos, bad, quick)) return quick;
+// transmission of cell (fi, fk); every cell here is past the wrapped one
+__device__ __forceinline__ float map_value(const BeamDev& b, int fi, int fk) {
+  const int r = fi + 1999 - b.br0, c = fk + 1999 - b.bc0;
+  return ((unsigned)r < (unsigned)b.rlim && (unsigned)c < (unsigned)b.clim) ? __ldg(b.block + (size_t)r * b.bcols + c)
+                                                                            : 0.0f;
+}
+
+// v / n correctly rounded for float32 v and n = S^3 <= 4096 without the
+// division subroutine: product with the rounded reciprocal and one residual
+// step (equal to the quotient for every float32 significand and S = 1..16,
+// tests/test_lattice_cpu.py)
+__device__ __forceinline__ double div_count(float v, double n, double inv_n) {
+  const double q = dmul((double)v, inv_n);
+  return __fma_rn(__fma_rn(-n, q, (double)v), inv_n, q);
+}
+
+// Blocked fraction (float64, the reference's sum acc + v / S^3 over ix, iy,
+// iz) of one voxel, every lane its own voxel.
+//
+// A uniform crop (jaws): a voxel whose samples all lie inside, or all outside,
+// the open rectangle is decided by its centre and the lattice's bound; the
+// others count their open samples by the signed distance to the rectangle
+// (about 15 instructions a sample), and the sum of n ones and S^3 - n zeros
+// is the n-th partial sum of 1 / S^3.  A map with other values looks every
+// sample's cell up.  A sample within SAMPLE_DELTA cells of a cell (or
+// rectangle) edge that matters takes the exact float64 mirror.
+//
+// Both were bound by instruction issue: the field-edge voxels of a jaw field
+// were classified one per warp round, 27 lanes each (a chunk of 32 edge voxels
+// took 32 rounds), and a map's voxels went through those rounds and then again
+// through a per-lane loop with a float64 division per change of value.
+// Measured, whole call: nine MLC beams on 140 x 101 x 112 9425 -> 5060 us, one
+// 5 x 5 cm beam on 128^3 227 -> 194 us.
+__device__ __forceinline__ double blocked_fraction(const BeamDev& b, const GridDev& g, int S, const float* pos,
+                                                   int& bad) {
+  Centre c;
+  if (!lattice_centre(b, pos, c)) return blocked_general(b, g, S, pos, bad);
+  // signed distances (cells) of the centre outside the crop's open cells
+  const float du = fabsf(c.u - b.uc) - b.uh, dw = fabsf(c.w - b.wc) - b.wh;
+  if (du > c.mu || dw > c.mw) return 0.0;
   float off[3];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) off[k] = fdiv(g.spacing[k], 3.0f);
-  int n_one = 0;
-  bool other = false;
-  // a rolled loop: one copy of the sample code keeps the kernel inside the
-  // instruction cache (the float32 offsets only steer the classification,
-  // whose ambiguous samples are recomputed exactly from ix, iy, iz)
-#pragma unroll 1
-  for (int sidx = 0; sidx < 27; ++sidx) {
-    const float v = sample_of(b, g, pos, off, sidx, bad);
-    n_one += v == 1.0f ? 1 : 0;
-    other |= v != 0.0f && v != 1.0f;
+  for (int k = 0; k < 3; ++k) off[k] = fdiv(g.spacing[k], (float)S);
+  if (b.uniform) {
+    if (du < -c.mu && dw < -c.mw) return c_unit_sum[S];
+    int n = 0;
+    for_samples(b, off, S, c, [&](int ix, int iy, int iz, float u, float w) {
+      const float d = fmaxf(fabsf(u - b.uc) - b.uh, fabsf(w - b.wc) - b.wh);
+      if (fabsf(d) > SAMPLE_DELTA)
+        n += d < 0.0f ? 1 : 0;
+      else
+        n += sample_exact(b, g, pos, off, ix, iy, iz, bad) == 1.0f ? 1 : 0;
+    });
+    if (S == 3) return c_unit_partial[n];
+    const double q = ddiv(1.0, (double)(S * S * S));
+    double acc = 0.0;
+    for (int i = 0; i < n; ++i) acc = dadd(acc, q);
+    return acc;
   }
-  if (!other) return c_unit_partial[n_one];
-  return blocked_general(b, g, 3, pos, bad);
-}
-
-// blocked_fraction for the voxels of a converged warp: the quick decisions
-// per lane, then, for each voxel that needs its samples classified, lanes
-// 0..26 classify one sample each (a warp's field-edge voxels cost one sample
-// time each instead of the whole warp running 27).  have: the lane holds a
-// voxel at pos.
-__device__ __forceinline__ double blocked_fraction_warp(const BeamDev& b, const GridDev& g, int S, bool have,
-                                                        const float* pos, int& bad) {
-  double out = 0.0;
-  const bool need = have && !blocked_quick(b, g, S, pos, bad, out);
-  unsigned m = __ballot_sync(0xffffffffu, need);
-  if (!m) return out;
-  const int lane = threadIdx.x & 31;
-  float off[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) off[k] = fdiv(g.spacing[k], 3.0f);
-  int n_one = 0;
-  bool other = false;
-  while (m) {
-    const int src = __ffs(m) - 1;
-    m &= m - 1;
-    float p[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) p[k] = __shfl_sync(0xffffffffu, pos[k], src);
-    int sbad = 0;
-    const float v = lane < 27 ? sample_of(b, g, p, off, lane, sbad) : 0.0f;
-    const unsigned ones = __ballot_sync(0xffffffffu, v == 1.0f);
-    const unsigned oth = __ballot_sync(0xffffffffu, v != 0.0f && v != 1.0f);
-    const unsigned bd = __ballot_sync(0xffffffffu, sbad != 0);
-    if (lane == src) {
-      n_one = __popc(ones);
-      other = oth != 0;
-      if (bd) bad = 1;
+  const double count = (double)(S * S * S), inv = ddiv(1.0, count);
+  double acc = 0.0, q = 0.0;
+  float last = 0.0f;
+  for_samples(b, off, S, c, [&](int ix, int iy, int iz, float u, float w) {
+    const int i0 = floor_int(u - SAMPLE_DELTA), i1 = floor_int(u + SAMPLE_DELTA);
+    const int k0 = floor_int(w - SAMPLE_DELTA), k1 = floor_int(w + SAMPLE_DELTA);
+    float v = map_value(b, i0, k0);
+    if (i0 != i1 || k0 != k1) {
+      const float v1 = map_value(b, i1, k0), v2 = map_value(b, i0, k1), v3 = map_value(b, i1, k1);
+      if (v1 != v || v2 != v || v3 != v) v = sample_exact(b, g, pos, off, ix, iy, iz, bad);
     }
-  }
-  if (need) out = other ? blocked_general(b, g, 3, pos, bad) : c_unit_partial[n_one];
-  return out;
+    if (v != last) {
+      last = v;
+      q = div_count(v, count, inv);
+    }
+    if (v != 0.0f) acc = dadd(acc, q);
+  });
+  return acc;
 }
 
 // ------------------------------------------------------------------ DDA --
@@ -555,7 +560,7 @@ __global__ void __launch_bounds__(256) cull_batch_kernel(const PrologueBeam* __r
 // radiological depth, oad, fluence, softening/horn and TERMA; TERMA support
 // box for the cone stage.
 // Entry e of a beam's list of count voxels; every lane of the warp calls it
-// (the blocking classification and the box reduction are warp-wide).
+// (the box reduction is warp-wide).
 __device__ __forceinline__ void terma_entry(const float* __restrict__ rho, const GridDev& g, const BeamDev& b,
                                             const SettingsDev& s, float* __restrict__ T, const Inter& inter,
                                             int all_voxels, int count, int e, const int* __restrict__ list_v,
@@ -575,9 +580,8 @@ __device__ __forceinline__ void terma_entry(const float* __restrict__ rho, const
       pos[1] = voxel_centre(g.origin[1], g.spacing[1], y);
       pos[2] = voxel_centre(g.origin[2], g.spacing[2], z);
     }
-    // (every lane of the warp: the sample classification is shared)
-    const double blocked = blocked_fraction_warp(b, g, s.samples, live, pos, bad);
     if (live) {
+      const double blocked = blocked_fraction(b, g, s.samples, pos, bad);
       if (inter.blocked) inter.blocked[v] = blocked;
       if (blocked == 0.0 && !all_voxels) {
         if (inter.terma) inter.terma[v] = 0.0f;
@@ -838,6 +842,12 @@ void upload_unit_partials() {
   const double q = 1.0 / 27.0;
   for (int i = 1; i < 28; ++i) p[i] = p[i - 1] + q;
   cudaMemcpyToSymbol(c_unit_partial, p, sizeof(p));
+  double full[17] = {0.0};
+  for (int S = 1; S <= 16; ++S) {
+    const double w = 1.0 / (double)(S * S * S);
+    for (int i = 0; i < S * S * S; ++i) full[S] += w;
+  }
+  cudaMemcpyToSymbol(c_unit_sum, full, sizeof(full));
 }
 
 void launch_prologue(const float* rho, const GridDev& g, const BeamDev& b, const SettingsDev& s, float* T,
