@@ -29,7 +29,8 @@ constexpr float SAMPLE_DELTA = 0.05f;   // cells (0.1 mm) of float32 slack
 // partial sums 0, 1/27, 1/27+1/27, ... accumulated in float64 as the
 // reference does for a block value of exactly 1.0 and 3x3x3 samples
 __constant__ double c_unit_partial[28];
-// the same sums over all S^3 sub-samples, S = 1..16
+// for S = 1..16 sub-samples per axis: 1 / S^3, and the sum of S^3 such terms
+__constant__ double c_inv_count[17];
 __constant__ double c_unit_sum[17];
 
 // --------------------------------------------------------- block lookup --
@@ -274,8 +275,9 @@ __device__ __forceinline__ float map_value(const BeamDev& b, int fi, int fk) {
 // v / n correctly rounded for float32 v and n = S^3 <= 4096 without the
 // division subroutine: product with the rounded reciprocal and one residual
 // step (equal to the quotient for every float32 significand and S = 1..16,
-// tests/test_lattice_cpu.py)
+// tests/test_lattice_cpu.py; infinities and NaN take the division)
 __device__ __forceinline__ double div_count(float v, double n, double inv_n) {
+  if (!(fabsf(v) <= 3.4028234e38f)) return ddiv((double)v, n);
   const double q = dmul((double)v, inv_n);
   return __fma_rn(__fma_rn(-n, q, (double)v), inv_n, q);
 }
@@ -318,12 +320,12 @@ __device__ __forceinline__ double blocked_fraction(const BeamDev& b, const GridD
         n += sample_exact(b, g, pos, off, ix, iy, iz, bad) == 1.0f ? 1 : 0;
     });
     if (S == 3) return c_unit_partial[n];
-    const double q = ddiv(1.0, (double)(S * S * S));
+    const double q = c_inv_count[S];
     double acc = 0.0;
     for (int i = 0; i < n; ++i) acc = dadd(acc, q);
     return acc;
   }
-  const double count = (double)(S * S * S), inv = ddiv(1.0, count);
+  const double count = (double)(S * S * S), inv = c_inv_count[S];
   double acc = 0.0, q = 0.0;
   float last = 0.0f;
   for_samples(b, off, S, c, [&](int ix, int iy, int iz, float u, float w) {
@@ -769,19 +771,41 @@ __device__ int sample_beamlet(const BeamDev& b, const BeamletDev& bl, const Grid
   return beamlet_of(b, bl, fi, fk);
 }
 
+// Row (or column) of beamlets of one sub-sample coordinate: v is its cell
+// coordinate relative to the grid's first cell, n beamlets of `cell` cells.
+// -1 outside the grid; ambiguous (near an edge between beamlets or of the
+// grid, within SAMPLE_DELTA) sets amb.
+__device__ __forceinline__ int beamlet_index(float v, float cell, float inv_cell, int n, bool& amb) {
+  const float q = floorf(v * inv_cell), d = v - q * cell;
+  const bool in = q >= 0.0f && q < (float)n;
+  amb = amb || ((d < SAMPLE_DELTA || d > cell - SAMPLE_DELTA) && q >= -1.0f && q <= (float)n);
+  return in ? (int)q : -1;
+}
+
 // dL/dw for blocked(v) = sum_s w[beamlet(s)] / S^3 and T = blocked^2 * H
 // (fluence and TERMA each carry one factor of blocked): over the voxels of
 // the prologue's list with T != 0, g(v) = tbar(v) * 2 T(v) / blocked(v) is
 // spread over the beamlets of its S^3 sub-samples.  Per-CTA float64
 // histograms in shared memory, one global float64 add per touched beamlet.
-__global__ void __launch_bounds__(256) blocked_adjoint_kernel(GridDev g, BeamDev b, BeamletDev bl, int S,
-                                                              const float* __restrict__ T,
-                                                              const float* __restrict__ tbar,
-                                                              const int* __restrict__ list_count,
-                                                              const int* __restrict__ list_v,
-                                                              double* __restrict__ wbar, int* __restrict__ flags) {
+//
+// One voxel per lane, 32 consecutive entries of the list per warp.  A voxel
+// whose samples span at most 2 x 2 beamlets (beamlets wider than its shadow
+// on the block plane) counts its samples per beamlet in four byte fields, and
+// the warp adds each beamlet's total once: float64 adds in shared memory are
+// compare-and-swap loops, and a warp's voxels lie in the same few beamlets, so
+// one add per sample serialised 32 ways.  Smaller beamlets add per change of
+// beamlet.
+constexpr int ADJ_THREADS = 512;
+__global__ void __launch_bounds__(ADJ_THREADS) blocked_adjoint_kernel(GridDev g, BeamDev b, BeamletDev bl, int S,
+                                                                      const float* __restrict__ T,
+                                                                      const float* __restrict__ tbar,
+                                                                      const int* __restrict__ list_count,
+                                                                      const int* __restrict__ list_v,
+                                                                      double* __restrict__ wbar,
+                                                                      int* __restrict__ flags) {
   extern __shared__ double hist[];
-  const int nb = bl.rows * bl.cols;
+  const unsigned full = 0xffffffffu;
+  const int nb = bl.rows * bl.cols, lane = threadIdx.x & 31;
   for (int i = threadIdx.x; i < nb; i += blockDim.x) hist[i] = 0.0;
   __syncthreads();
   const int count = *list_count;
@@ -790,33 +814,105 @@ __global__ void __launch_bounds__(256) blocked_adjoint_kernel(GridDev g, BeamDev
 #pragma unroll
   for (int k = 0; k < 3; ++k) off[k] = fdiv(g.spacing[k], (float)S);
   const double inv = 1.0 / ((double)S * (double)S * (double)S);
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < count; e += gridDim.x * blockDim.x) {
-    const int v = list_v[e];
-    const int z = v % g.n[2];
-    const int r = v / g.n[2];
-    const int y = r % g.n[1];
-    const int x = r / g.n[1];
-    const float t = T[((size_t)x * g.n[1] + y) * g.zp + z];
-    const float tb = tbar[v];
-    if (t == 0.0f || tb == 0.0f) continue;
-    float pos[3];
-    pos[0] = voxel_centre(g.origin[0], g.spacing[0], x);
-    pos[1] = voxel_centre(g.origin[1], g.spacing[1], y);
-    pos[2] = voxel_centre(g.origin[2], g.spacing[2], z);
-    const double blocked = blocked_fraction(b, g, S, pos, bad);
-    if (!(blocked > 0.0)) continue;
-    const double gv = (double)tb * 2.0 * (double)t / blocked * inv;
-    for (int ix = 0; ix < S; ++ix)
-      for (int iy = 0; iy < S; ++iy)
-        for (int iz = 0; iz < S; ++iz) {
-          const float rx = off[0] * ((float)ix + 0.5f) - g.spacing[0] * 0.5f;
-          const float ry = off[1] * ((float)iy + 0.5f) - g.spacing[1] * 0.5f;
-          const float rz = off[2] * ((float)iz + 0.5f) - g.spacing[2] * 0.5f;
-          const int id = sample_beamlet(b, bl, g, pos, off, rx, ry, rz, ix, iy, iz, bad);
-          if (id >= 0) atomicAdd(hist + id, gv);
+  const float cr = (float)bl.cell_rows, cc = (float)bl.cell_cols;
+  const float icr = 1.0f / cr, icc = 1.0f / cc;
+  // cell coordinate of the beamlet grid's first row and column
+  const float u0 = (float)(bl.r0 - 1999), w0 = (float)(bl.c0 - 1999);
+  // the grid ends where the map does: its last row and column are read by the wrapped index only
+  const bool whole = bl.r0 + bl.rows * bl.cell_rows <= 3999 && bl.c0 + bl.cols * bl.cell_cols <= 3999;
+  const int stride = gridDim.x * blockDim.x;
+  const int rounds = (count + stride - 1) / stride;
+  for (int it = 0; it < rounds; ++it) {
+    const int e = it * stride + blockIdx.x * blockDim.x + threadIdx.x;
+    float t = 0.0f, tb = 0.0f, pos[3] = {0.0f, 0.0f, 0.0f};
+    if (e < count) {
+      const int v = list_v[e];
+      const int z = v % g.n[2];
+      const int r = v / g.n[2];
+      const int y = r % g.n[1];
+      const int x = r / g.n[1];
+      t = T[((size_t)x * g.n[1] + y) * g.zp + z];
+      tb = tbar[v];
+      pos[0] = voxel_centre(g.origin[0], g.spacing[0], x);
+      pos[1] = voxel_centre(g.origin[1], g.spacing[1], y);
+      pos[2] = voxel_centre(g.origin[2], g.spacing[2], z);
+    }
+    unsigned cnt = 0;      // samples in beamlets (a, c), (a, c + 1), (a + 1, c), (a + 1, c + 1), a byte each
+    int id0 = 0;           // beamlet (a, c), which may lie outside the grid
+    double gv = 0.0;
+    if (t != 0.0f && tb != 0.0f) {
+      const double blocked = blocked_fraction(b, g, S, pos, bad);
+      Centre c;
+      if (blocked > 0.0) {
+        gv = (double)tb * 2.0 * (double)t / blocked * inv;
+        const bool lat = whole && lattice_centre(b, pos, c);
+        int a = 0, k = 0;
+        bool four = false;
+        if (lat) {
+          a = floor_int((c.u - c.mu - u0) * icr - 1e-3f);
+          k = floor_int((c.w - c.mw - w0) * icc - 1e-3f);
+          four = S <= 6 && floor_int((c.u + c.mu - u0) * icr + 1e-3f) <= a + 1 &&
+                 floor_int((c.w + c.mw - w0) * icc + 1e-3f) <= k + 1;
+          id0 = a * bl.cols + k;
         }
+        if (lat) {
+          int cur = -1, n = 0;
+          for_samples(b, off, S, c, [&](int ix, int iy, int iz, float u, float w) {
+            bool amb = false;
+            int i = beamlet_index(u - u0, cr, icr, bl.rows, amb), j = beamlet_index(w - w0, cc, icc, bl.cols, amb);
+            if (amb) {
+              int fi, fk;
+              int id = -1;
+              if (sample_cell_exact(b, g, pos, off, ix, iy, iz, bad, fi, fk)) id = beamlet_of(b, bl, fi, fk);
+              i = id < 0 ? -1 : id / bl.cols;
+              j = id < 0 ? -1 : id - i * bl.cols;
+            }
+            if (i < 0 || j < 0) return;
+            if (four && (unsigned)(i - a) < 2u && (unsigned)(j - k) < 2u) {
+              cnt += 1u << (8 * (2 * (i - a) + (j - k)));
+            } else {
+              const int id = i * bl.cols + j;
+              if (id != cur) {
+                if (n) atomicAdd(hist + cur, gv * (double)n);
+                cur = id;
+                n = 0;
+              }
+              ++n;
+            }
+          });
+          if (n) atomicAdd(hist + cur, gv * (double)n);
+        } else {
+          for (int ix = 0; ix < S; ++ix)
+            for (int iy = 0; iy < S; ++iy)
+              for (int iz = 0; iz < S; ++iz) {
+                const float rx = off[0] * ((float)ix + 0.5f) - g.spacing[0] * 0.5f;
+                const float ry = off[1] * ((float)iy + 0.5f) - g.spacing[1] * 0.5f;
+                const float rz = off[2] * ((float)iz + 0.5f) - g.spacing[2] * 0.5f;
+                const int id = sample_beamlet(b, bl, g, pos, off, rx, ry, rz, ix, iy, iz, bad);
+                if (id >= 0) atomicAdd(hist + id, gv);
+              }
+        }
+      }
+    }
+    // the warp's totals, one add per beamlet and field (only beamlets of the grid hold counts)
+#pragma unroll 1
+    for (int f = 0; f < 4; ++f) {
+      const int n = (int)((cnt >> (8 * f)) & 255u);
+      const int id = id0 + (f >> 1) * bl.cols + (f & 1);
+      unsigned todo = __ballot_sync(full, n > 0);
+      while (todo) {
+        const int lead = __ffs(todo) - 1;
+        const int lid = __shfl_sync(full, id, lead);
+        const bool mine = n > 0 && id == lid;
+        double sum = mine ? gv * (double)n : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(full, sum, o);
+        if (lane == lead) atomicAdd(hist + lid, sum);
+        todo &= ~__ballot_sync(full, mine);
+      }
+    }
   }
-  if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(flags, FLAG_PARALLEL_RAY);
+  if (__any_sync(full, bad) && lane == 0) atomicOr(flags, FLAG_PARALLEL_RAY);
   __syncthreads();
   for (int i = threadIdx.x; i < nb; i += blockDim.x)
     if (hist[i] != 0.0) atomicAdd(wbar + i, hist[i]);
@@ -832,7 +928,7 @@ cudaError_t launch_blocked_adjoint(const GridDev& g, const BeamDev& b, const Bea
                                          (int)smem);
     if (e != cudaSuccess) return e;
   }
-  blocked_adjoint_kernel<<<n_sm * 2, 256, smem, st>>>(g, b, bl, S, T, tbar, list_count, list_v, wbar, flags);
+  blocked_adjoint_kernel<<<n_sm * 2, ADJ_THREADS, smem, st>>>(g, b, bl, S, T, tbar, list_count, list_v, wbar, flags);
   return cudaGetLastError();
 }
 
@@ -842,11 +938,12 @@ void upload_unit_partials() {
   const double q = 1.0 / 27.0;
   for (int i = 1; i < 28; ++i) p[i] = p[i - 1] + q;
   cudaMemcpyToSymbol(c_unit_partial, p, sizeof(p));
-  double full[17] = {0.0};
+  double full[17] = {0.0}, inv[17] = {0.0};
   for (int S = 1; S <= 16; ++S) {
-    const double w = 1.0 / (double)(S * S * S);
-    for (int i = 0; i < S * S * S; ++i) full[S] += w;
+    inv[S] = 1.0 / (double)(S * S * S);
+    for (int i = 0; i < S * S * S; ++i) full[S] += inv[S];
   }
+  cudaMemcpyToSymbol(c_inv_count, inv, sizeof(inv));
   cudaMemcpyToSymbol(c_unit_sum, full, sizeof(full));
 }
 

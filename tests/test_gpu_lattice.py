@@ -1,8 +1,12 @@
-"""GPU: the blocked fraction's lattice path, where it can go wrong.
+"""GPU: the blocked fraction's lattice path and the beamlet adjoint's two ways
+of adding, where they can go wrong.
 
 * blocked is bit-exact against the float32-mirrored oracle for 1 to 5
   sub-samples per axis, for a jaw opening, a map of graded values and a map
   open to its last row and column (which the wrapped index also reads).
+* The gradient of small beamlets, summed over the coarse beamlet that holds
+  them, is the coarse beamlet's: the same samples through the per-change adds
+  and through the per-warp byte counts.
 """
 import numpy as np
 import pytest
@@ -53,3 +57,26 @@ def test_blocked_bitexact(settings, oracle_lib, kind, samples):
     ref = oracle_lib.prologue(src, blk, ph, s, oracle_lib.MODE_F32)["blocked"]
     assert (ref > 0).any()
     assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("coarse,cell,fine", [(8, 50, 10), (4, 25, 25), (6, 21, 3)])
+def test_fine_beamlets_sum_to_coarse_ones(settings, coarse, cell, fine):
+    import torch
+    from conehead_gb300.adjoint import BeamletDose, BeamletGrid
+    from conehead_gb300.conehead import engine
+    eng = engine(0)
+    ph = _phantom((40, 37, 30), (0.25, 0.25, 0.25))
+    src = _source(61.0, 13.0)
+    g = torch.Generator().manual_seed(coarse)
+    w = torch.rand((coarse, coarse), generator=g) + 0.1
+    up = torch.randn(tuple(ph.size), generator=g).cuda()
+    r0 = 2000 - coarse * cell // 2
+    big = BeamletDose(eng, ph, src, BeamletGrid(coarse, coarse, cell, r0=r0, c0=r0), settings)
+    k = fine
+    small = BeamletDose(eng, ph, src, BeamletGrid(coarse * k, coarse * k, cell // k, r0=r0, c0=r0), settings)
+    a = big.backward(up, weights=w.cuda()).double()
+    b = small.backward(up, weights=w.cuda().repeat_interleave(k, 0).repeat_interleave(k, 1)).double()
+    b = b.reshape(coarse, k, coarse, k).sum((1, 3))
+    assert float(a.abs().max()) > 0
+    # float32 stores of the fine gradients: 2^-24 of each, k^2 of them
+    assert float((a - b).abs().max()) <= 2e-6 * float(a.abs().max())
