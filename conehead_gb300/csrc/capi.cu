@@ -134,6 +134,7 @@ struct ch_plan {
   bool have_kernel = false;
   int n_phi = 0, n_r = 0, n_theta = 0;
   DevBuf K, theta, phi;
+  DevBuf K2;                 // K as float32 pairs (radiological scatter)
   std::vector<float> h_theta, h_phi;   // the direction tables the stencils were built from
   StencilSet st;
   StencilSet st_adj;         // the same walks mirrored (offsets and directions negated): the transposed cone
@@ -159,7 +160,7 @@ struct ch_plan {
     for (int i = 0; i < 2; ++i)
       if (rec_pending[i] && ev_rec[i]) cudaEventSynchronize(ev_rec[i]);
     spec.clear();
-    for (DevBuf* b : {&K, &theta, &phi, &T, &aabb, &counters, &ranges, &cranges, &cone_beams, &range_beams, &list_v,
+    for (DevBuf* b : {&K, &K2, &theta, &phi, &T, &aabb, &counters, &ranges, &cranges, &cone_beams, &range_beams, &list_v,
                       &spec_work, &pro_beams, &spec_tw, &adj_in, &adj_out, &adj_w})
       b->release();
     for (StencilSet* S : {&st, &st_adj})
@@ -1307,7 +1308,8 @@ ch_status run_group(ch_plan* P, int n, const ch_grid* grids, const float* const*
       if (radiological)
         launch_scatter_radiological(S.T + J.t_off, J.rho, J.g.n, J.g.zp, J.g.swap_xy, B.U, D.tap_base, D.tap_len,
                                     D.offs, D.tvals, B.set->walk_row.as<int>(), B.set->walk_mult.as<int>(),
-                                    P->K.as<double>(), P->n_r, J.dose, s);
+                                    P->K2.as<float2>(), P->n_r, S.aabb + 8 * i + 6, S.list_v + J.l_off, P->n_sm,
+                                    J.dose, s);
       else
         launch_scatter(S.T + J.t_off, J.g.n, J.g.zp, B.U, D.tap_base, D.tap_len, D.offs, D.taps, J.dose, s);
       CH_CUDA(cudaGetLastError());
@@ -1462,12 +1464,16 @@ ch_status ch_plan_set_kernel(ch_plan* P, const ch_kernel* k) {
                          std::equal(k->theta, k->theta + k->n_theta, P->h_theta.begin()) &&
                          std::equal(k->phi, k->phi + k->n_phi, P->h_phi.begin());
   CH_CUDA(P->K.ensure((size_t)k->n_phi * k->n_r * sizeof(double)));
+  CH_CUDA(P->K2.ensure((size_t)k->n_phi * k->n_r * sizeof(float2)));
   CH_CUDA(P->theta.ensure((size_t)k->n_theta * sizeof(float)));
   CH_CUDA(P->phi.ensure((size_t)k->n_phi * sizeof(float)));
   CH_CUDA(cudaDeviceSynchronize());   // no call of this plan may still read the old tables
   CH_CUDA(cudaMemcpy(P->K.p, k->cum, (size_t)k->n_phi * k->n_r * sizeof(double), cudaMemcpyHostToDevice));
   CH_CUDA(cudaMemcpy(P->theta.p, k->theta, (size_t)k->n_theta * sizeof(float), cudaMemcpyHostToDevice));
   CH_CUDA(cudaMemcpy(P->phi.p, k->phi, (size_t)k->n_phi * sizeof(float), cudaMemcpyHostToDevice));
+  launch_split_table(P->K.as<double>(), k->n_phi * k->n_r, P->K2.as<float2>(), nullptr);
+  CH_CUDA(cudaGetLastError());
+  CH_CUDA(cudaStreamSynchronize(nullptr));
   P->n_phi = k->n_phi;
   P->n_r = k->n_r;
   P->n_theta = k->n_theta;
@@ -2031,7 +2037,7 @@ ch_status ch_plan_prepare(ch_plan* P, const ch_grid* grid, void* stream) {
 
 ch_status ch_plan_memory(ch_plan* P, size_t* tables, size_t* scratch) {
   if (!P) return fail(CH_ERR_INVALID_ARG, "plan is NULL");
-  size_t b = P->K.bytes + P->theta.bytes + P->phi.bytes;
+  size_t b = P->K.bytes + P->K2.bytes + P->theta.bytes + P->phi.bytes;
   for (const StencilSet* S : {&P->st, &P->st_adj}) b += S->bytes();
   for (const auto& e : P->spec) b += e->shat.bytes;
   b += P->spec_tw.bytes;

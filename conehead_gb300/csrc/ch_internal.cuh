@@ -331,8 +331,10 @@ void launch_stencil(const float* theta, int n_theta, const float* phi, int n_phi
                     int* len, float* dirs, const ConeFrame& frame, cudaStream_t st);
 void launch_scatter_radiological(const float* T, const float* rho, const int* n, int zp, int swap_xy, int n_dirs,
                                  const int* tap_base, const int* tap_len, const short4* offs, const float* tvals,
-                                 const int* walk_row, const int* walk_mult, const double* K, int n_r, float* dose,
-                                 cudaStream_t st);
+                                 const int* walk_row, const int* walk_mult, const float2* K2, int n_r,
+                                 const int* list_count, const int* list_v, int n_sm, float* dose, cudaStream_t st);
+// K as float32 pairs (hi + lo), read by the radiological scatter
+void launch_split_table(const double* K, int n, float2* out, cudaStream_t st);
 void launch_reweight(const double* K, int n_r, int n_walks, const int* tap_base, const int* tap_len,
                      const float* tvals, const int* walk_row, const int* walk_mult, int4* taps, const int* tap_run,
                      int4* runs, cudaStream_t st);
