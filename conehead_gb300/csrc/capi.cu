@@ -729,6 +729,22 @@ BeamDev make_beam(const ch_beam& in, const ch_grid& g, int samples) {
     b.lat_0 += h * std::fabs(b.m0f[k]);
     b.lat_2 += h * std::fabs(b.m2f[k]);
   }
+  // float32 error bounds of the projection (lattice_centre in prologue.cu)
+  double P = 0.0, P1 = 0.0, D = 0.0;
+  for (int c = 0; c < 8; ++c) {
+    double sum = 0.0, d2 = 0.0;
+    for (int k = 0; k < 3; ++k) {
+      const double p = (double)g.origin[k] + (((c >> k) & 1) ? g.n[k] - 0.5 : -0.5) * (double)g.spacing[k];
+      P = std::max(P, std::fabs(p));
+      sum += std::fabs(p);
+      d2 += (b.src[k] - p) * (b.src[k] - p);
+    }
+    P1 = std::max(P1, sum);
+    D = std::max(D, std::sqrt(d2));
+  }
+  const double ray = std::sqrt(3.0) * P + D + 8.0 * P1;
+  b.err_x = (float)(std::ldexp(1.0, -24) * (ray + 5.0 * std::max(std::fabs(m0S), std::fabs(m2S))));
+  b.err_n = (float)(std::ldexp(1.0, -24) * (ray + 5.0 * std::fabs(nS)));
   // map index r is read by cell r - 1999, cells -1999..1999 (the wrapped one aside)
   b.rlim = std::max(0, std::min(in.block_rows, 3999 - in.block_r0));
   b.clim = std::max(0, std::min(in.block_cols, 3999 - in.block_c0));

@@ -108,6 +108,7 @@ struct BeamDev {
   int lat;              // float64 source arrays: samples may be classified in float32
   int wraps;            // the crop holds the map's last row or column, which index -2000 reads
   float lat_n, lat_0, lat_2;   // largest |d nd|, |d x0|, |d x2| of a sub-sample from its voxel centre (cm)
+  float err_x, err_n;   // float32 error bounds of x0 and nd against the reference's ray (cm)
   float uc, uh, wc, wh; // the crop's cells, centre and half width along u (rows) and w (columns)
   int rlim, clim;       // crop rows and columns a lookup can reach without the wrap
   // fluence / TERMA

@@ -210,15 +210,28 @@ __device__ __noinline__ double blocked_general(const BeamDev& b, const GridDev& 
 struct Centre {
   float nd, x0, x2;     // the linear forms at the voxel centre
   float u, w, mu, mw;   // its cell coordinates, and how far a sub-sample's may be from them
+  float delta;          // bound of |float32 - reference| of a sample's cell coordinates
 };
 
 // Projects the voxel centre and bounds the sub-samples around it.  For an
 // offset of the lattice's box, |d nd| <= A = lat_n, |d x0| <= B = lat_0, so
 //   |d(K x0 / nd)| <= |K| (B + |x0 / nd| A) / (|nd| - A).
-// False when a sub-sample may lie closer to the source plane than 0.2 |K|
-// (the float32 error bound SAMPLE_DELTA assumes a magnification below 5) or
+// False when a sub-sample may lie closer to the source plane than 0.2 |K| or
 // may read the wrapped cell -2000 of a crop that holds the map's last row or
 // column: those voxels, and float32 source arrays, take blocked_general.
+//
+// delta bounds the difference between a float32 cell coordinate and the
+// reference's, whose ray and plane point are float32 stores as well.  With
+// P the largest |coordinate| of the grid, P1 the largest sum of three, D the
+// largest distance to the source and m the magnification |K / nd|, in units of
+// 2^-24 (a rounding of 1): the reference's sample point and ray are off by at
+// most sqrt(3) P + D, which moves its plane point by m (1 + lat) times that;
+// here x0 is off by 8 P1 + 5 |m0.S| (inputs, products, sums, lattice steps)
+// and nd by 8 P1 + 5 |n.S|, which moves K x0 / nd by m and m lat times that.
+// The plane point's own roundings, the quotient and the scaling by 100 stay
+// below 0.002 cells within the map.  About 0.008 cells on a 40 cm grid: a
+// seventh of the samples of a fixed 0.05 take the float64 mirror, which cost
+// a map with graded cells (MLC leaf edges) two thirds of its TERMA launch.
 __device__ __forceinline__ bool lattice_centre(const BeamDev& b, const float* pos, Centre& c) {
   if (!b.lat) return false;
   c.nd = b.a_nS - (b.vyf[0] * pos[0] + b.vyf[1] * pos[1] + b.vyf[2] * pos[2]);
@@ -230,8 +243,10 @@ __device__ __forceinline__ bool lattice_centre(const BeamDev& b, const float* po
   const float inv = __fdividef(1.0f, c.nd), mag = __fdividef(fabsf(K), near);
   c.u = K * inv * c.x0 + 100.0f * b.a_c0;
   c.w = K * inv * c.x2 + 100.0f * b.a_c2;
-  c.mu = mag * (b.lat_0 + fabsf(c.x0 * inv) * b.lat_n) + SAMPLE_DELTA;
-  c.mw = mag * (b.lat_2 + fabsf(c.x2 * inv) * b.lat_n) + SAMPLE_DELTA;
+  const float l0 = fabsf(c.x0 * inv), l2 = fabsf(c.x2 * inv);
+  c.delta = mag * (b.err_x + (fmaxf(l0, l2) + 0.01f) * b.err_n) + 0.002f;
+  c.mu = mag * (b.lat_0 + l0 * b.lat_n) + c.delta;
+  c.mw = mag * (b.lat_2 + l2 * b.lat_n) + c.delta;
   return !b.wraps || (c.u - c.mu > -1999.0f && c.w - c.mw > -1999.0f);
 }
 
@@ -290,8 +305,8 @@ __device__ __forceinline__ double div_count(float v, double n, double inv_n) {
 // others count their open samples by the signed distance to the rectangle
 // (about 15 instructions a sample), and the sum of n ones and S^3 - n zeros
 // is the n-th partial sum of 1 / S^3.  A map with other values looks every
-// sample's cell up.  A sample within SAMPLE_DELTA cells of a cell (or
-// rectangle) edge that matters takes the exact float64 mirror.
+// sample's cell up.  A sample within delta of a cell (or rectangle) edge that
+// matters takes the exact float64 mirror.
 //
 // Both were bound by instruction issue: the field-edge voxels of a jaw field
 // were classified one per warp round, 27 lanes each (a chunk of 32 edge voxels
@@ -314,7 +329,7 @@ __device__ __forceinline__ double blocked_fraction(const BeamDev& b, const GridD
     int n = 0;
     for_samples(b, off, S, c, [&](int ix, int iy, int iz, float u, float w) {
       const float d = fmaxf(fabsf(u - b.uc) - b.uh, fabsf(w - b.wc) - b.wh);
-      if (fabsf(d) > SAMPLE_DELTA)
+      if (fabsf(d) > c.delta)
         n += d < 0.0f ? 1 : 0;
       else
         n += sample_exact(b, g, pos, off, ix, iy, iz, bad) == 1.0f ? 1 : 0;
@@ -329,8 +344,8 @@ __device__ __forceinline__ double blocked_fraction(const BeamDev& b, const GridD
   double acc = 0.0, q = 0.0;
   float last = 0.0f;
   for_samples(b, off, S, c, [&](int ix, int iy, int iz, float u, float w) {
-    const int i0 = floor_int(u - SAMPLE_DELTA), i1 = floor_int(u + SAMPLE_DELTA);
-    const int k0 = floor_int(w - SAMPLE_DELTA), k1 = floor_int(w + SAMPLE_DELTA);
+    const int i0 = floor_int(u - c.delta), i1 = floor_int(u + c.delta);
+    const int k0 = floor_int(w - c.delta), k1 = floor_int(w + c.delta);
     float v = map_value(b, i0, k0);
     if (i0 != i1 || k0 != k1) {
       const float v1 = map_value(b, i1, k0), v2 = map_value(b, i0, k1), v3 = map_value(b, i1, k1);
@@ -773,12 +788,12 @@ __device__ int sample_beamlet(const BeamDev& b, const BeamletDev& bl, const Grid
 
 // Row (or column) of beamlets of one sub-sample coordinate: v is its cell
 // coordinate relative to the grid's first cell, n beamlets of `cell` cells.
-// -1 outside the grid; ambiguous (near an edge between beamlets or of the
-// grid, within SAMPLE_DELTA) sets amb.
-__device__ __forceinline__ int beamlet_index(float v, float cell, float inv_cell, int n, bool& amb) {
+// -1 outside the grid; within delta of an edge between beamlets or of the
+// grid sets amb.
+__device__ __forceinline__ int beamlet_index(float v, float cell, float inv_cell, int n, float delta, bool& amb) {
   const float q = floorf(v * inv_cell), d = v - q * cell;
   const bool in = q >= 0.0f && q < (float)n;
-  amb = amb || ((d < SAMPLE_DELTA || d > cell - SAMPLE_DELTA) && q >= -1.0f && q <= (float)n);
+  amb = amb || ((d < delta || d > cell - delta) && q >= -1.0f && q <= (float)n);
   return in ? (int)q : -1;
 }
 
@@ -859,7 +874,8 @@ __global__ void __launch_bounds__(ADJ_THREADS) blocked_adjoint_kernel(GridDev g,
           int cur = -1, n = 0;
           for_samples(b, off, S, c, [&](int ix, int iy, int iz, float u, float w) {
             bool amb = false;
-            int i = beamlet_index(u - u0, cr, icr, bl.rows, amb), j = beamlet_index(w - w0, cc, icc, bl.cols, amb);
+            int i = beamlet_index(u - u0, cr, icr, bl.rows, c.delta, amb);
+            int j = beamlet_index(w - w0, cc, icc, bl.cols, c.delta, amb);
             if (amb) {
               int fi, fk;
               int id = -1;

@@ -6,10 +6,16 @@
   float64 form (``kernel_index_f32``), also one ulp beside every index's edge.
 * The float32 difference of two table entries held as float32 pairs is the
   float64 difference rounded once (``pair_diff``), up to one ulp.
+* A sub-sample's float32 cell coordinates, stepped along the lattice, stay
+  within ``lattice_centre``'s bound of the reference's (a float32 sample point,
+  ray and plane point, float64 in between).
 """
 import subprocess
 
 import numpy as np
+import pytest
+
+from conehead_gb300.source import Source
 
 F = np.float32
 
@@ -77,3 +83,59 @@ def test_difference_of_pairs(settings):
     got = d + (err + (l1 - l0))
     ref = K[row, b] - K[row, a]
     assert np.all(np.abs(got.astype(np.float64) - ref) <= np.spacing(np.abs(ref).astype(F)))
+
+
+@pytest.mark.parametrize("seed", range(12))
+def test_projection_bound(seed):
+    rng = np.random.default_rng(seed)
+    src = Source()
+    src.gantry, src.collimator = float(rng.uniform(0, 360)), float(rng.uniform(0, 90))
+    n = rng.integers(24, 260, 3)
+    sp = rng.choice([0.1, 0.2, 0.25, 0.3, 0.5], 3).astype(F)
+    org = (-(n - 1) * sp / 2 + rng.uniform(-8, 8, 3)).astype(F)
+    S = int(rng.integers(1, 6))
+    pos, vy, m = np.asarray(src.position, float), np.asarray(src.v_y, float), np.asarray(src.transform, float)
+    srcf = pos.astype(F).astype(float)
+    vyw = (vy[0] * srcf[0] + vy[1] * srcf[1]) + vy[2] * srcf[2]
+    # constants of the beam
+    corners = np.array([[org[k] + (n[k] - 0.5 if c >> k & 1 else -0.5) * float(sp[k]) for k in range(3)]
+                        for c in range(8)])
+    P, P1 = np.abs(corners).max(), np.abs(corners).sum(1).max()
+    D = np.sqrt(((pos - corners) ** 2).sum(1)).max()
+    ray = np.sqrt(3) * P + D + 8 * P1
+    err_x = 2.0 ** -24 * (ray + 5 * max(abs(m[0] @ pos), abs(m[2] @ pos)))
+    err_n = 2.0 ** -24 * (ray + 5 * abs(vy @ pos))
+    h = 1.0001 * sp.astype(float) * (S - 1) / (2 * S)
+    lat_n = float(h @ np.abs(vy))
+    vyf, m0f, m2f = vy.astype(F), m[0].astype(F), m[2].astype(F)
+    K, c0, c2 = F(-vyw) * F(100), F(m[0] @ srcf) * F(100), F(m[2] @ srcf) * F(100)
+    vox = np.stack([rng.integers(0, k, 20000) for k in n], axis=1)
+    p = (org.astype(float) + sp.astype(float) * vox).astype(F)
+    nd = F(vy @ pos) - (vyf[0] * p[:, 0] + vyf[1] * p[:, 1] + vyf[2] * p[:, 2])
+    x0 = F(m[0] @ pos) - (m0f[0] * p[:, 0] + m0f[1] * p[:, 1] + m0f[2] * p[:, 2])
+    x2 = F(m[2] @ pos) - (m2f[0] * p[:, 0] + m2f[1] * p[:, 1] + m2f[2] * p[:, 2])
+    near = np.abs(nd) - F(lat_n)
+    ok = near > F(0.2) * abs(F(-vyw))
+    mag = np.abs(K) / near
+    lat = np.maximum(np.abs(x0 / nd), np.abs(x2 / nd))
+    delta = mag * (F(err_x) + (lat + F(0.01)) * F(err_n)) + F(0.002)
+    off = sp / F(S)
+    i = rng.integers(0, S, (len(p), 3))
+    mid = F(0.5) * F(S - 1)
+    a, b, c = nd, x0, x2
+    for k in range(3):
+        r = off[k] * (i[:, k].astype(F) - mid)
+        a, b, c = a - vyf[k] * r, b - m0f[k] * r, c - m2f[k] * r
+    si = K / a
+    u, w = si * b + c0, si * c + c2
+    # the reference's arithmetic
+    ps = np.stack([(((p[:, k].astype(float) - float(sp[k]) * 0.5) + float(off[k]) * 0.5) + float(off[k]) * i[:, k])
+                   .astype(F) for k in range(3)], axis=1)
+    rd = (pos - ps.astype(float)).astype(F).astype(float)
+    t = -vyw / ((vy[0] * rd[:, 0] + vy[1] * rd[:, 1]) + vy[2] * rd[:, 2])
+    pp = (srcf + t[:, None] * rd).astype(F).astype(float)
+    ref = [(((m[q][0] * pp[:, 0] + m[q][1] * pp[:, 1]) + m[q][2] * pp[:, 2]).astype(F) * F(100)) for q in (0, 2)]
+    on = ok & (np.abs(ref[0]) < 2200) & (np.abs(ref[1]) < 2200)
+    assert on.any()
+    worst = np.maximum(np.abs(u - ref[0]), np.abs(w - ref[1]))[on] / delta[on]
+    assert worst.max() < 0.8, worst.max()        # two more ulp of the fast division stay inside the rest
