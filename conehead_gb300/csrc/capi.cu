@@ -1188,6 +1188,7 @@ std::vector<PrologueBeam> make_prologue_records(const BatchPlan& B, const Scratc
     R.list_v = S.list_v + J.l_off;
     R.line_any = reinterpret_cast<unsigned char*>(S.list_v + J.f_off);
     R.zero_all = B.spectral ? 0 : 1;
+    R.box = B.spectral ? 0 : 1;
   }
   return pb;
 }
@@ -1227,8 +1228,8 @@ ch_status enqueue_batch(ch_plan* P, const BatchPlan& B, const Scratch& S, const 
       const BeamJob& J = B.jobs[i];
       int all = 0;
       const Inter in = make_inter(inter, all);
-      launch_prologue(J.rho, J.g, J.b, J.s, S.T + J.t_off, in, all, S.aabb + 8 * i, S.list_v + J.l_off, P->n_sm,
-                      flags, s, P->tuning.terma_ctas_per_sm);
+      launch_prologue(J.rho, J.g, J.b, J.s, S.T + J.t_off, in, all, S.aabb + 8 * i, !B.spectral,
+                      S.list_v + J.l_off, P->n_sm, flags, s, P->tuning.terma_ctas_per_sm);
       CH_CUDA(cudaGetLastError());
     }
   } else {
@@ -1311,9 +1312,8 @@ ch_status run_group(ch_plan* P, int n, const ch_grid* grids, const float* const*
       const BeamJob& J = B.jobs[i];
       int all = 0;
       const Inter in = make_inter(inter, all);
-      launch_prologue(J.rho, J.g, J.b, J.s, S.T + J.t_off, in, all, S.aabb + 8 * i, S.list_v + J.l_off, P->n_sm,
-                      flags, s,
-                      P->tuning.terma_ctas_per_sm);
+      launch_prologue(J.rho, J.g, J.b, J.s, S.T + J.t_off, in, all, S.aabb + 8 * i, false, S.list_v + J.l_off,
+                      P->n_sm, flags, s, P->tuning.terma_ctas_per_sm);
       CH_CUDA(cudaGetLastError());
     }
     CH_CUDA(cudaEventRecord(P->ev[1], s));
@@ -1608,7 +1608,7 @@ ch_status ch_dose_static(ch_plan* P, const ch_grid* grid, const float* rho, int 
   // aabb and the list count must start from their reset values; TERMA is
   // rewritten in full by the prologue and the range tables by range_kernel
   launch_init_scratch(aabb, 1, counters, s);
-  launch_prologue(rho, g, b, sd, T, Inter{}, 0, aabb, reinterpret_cast<int*>(base + o_lv), P->n_sm, flags, s,
+  launch_prologue(rho, g, b, sd, T, Inter{}, 0, aabb, true, reinterpret_cast<int*>(base + o_lv), P->n_sm, flags, s,
                   P->tuning.terma_ctas_per_sm);
   CH_CUDA(cudaGetLastError());
   CH_CUDA(cudaMemsetAsync(dose, 0, N * sizeof(float), s));
@@ -1842,7 +1842,8 @@ ch_status ch_dose_adjoint(ch_plan* P, const ch_grid* grid, const float* rho, int
   const SettingsDev sd = make_settings(*settings);
   launch_init_scratch(box, 2, counters, s);
   // forward prologue: TERMA, its box and the list of voxels the beam reaches
-  launch_prologue(rho, g, b, sd, P->T.as<float>(), Inter{}, 0, box, P->list_v.as<int>(), P->n_sm, flags, s, P->tuning.terma_ctas_per_sm);
+  launch_prologue(rho, g, b, sd, P->T.as<float>(), Inter{}, 0, box, !spec_batch(P, 1, grid), P->list_v.as<int>(),
+                  P->n_sm, flags, s, P->tuning.terma_ctas_per_sm);
   CH_CUDA(cudaGetLastError());
   // transposed cone: dL/dT = C^T dL/dD, only where TERMA is nonzero
   float* tbar = grad_terma ? grad_terma : P->adj_out.as<float>();

@@ -311,6 +311,7 @@ struct PrologueBeam {
   unsigned char* line_any;  // per (x, y) line: 1 when the line holds a listed voxel
   int zero_all;      // 1: zero TERMA on every line (the gather reads it anywhere);
                      // 0: only on lines with listed voxels (the spectral path reads line_any)
+  int box;           // 1: the gather needs the TERMA box
 };
 
 // ------------------------------------------------------------ launchers --
@@ -319,8 +320,8 @@ void upload_unit_partials();
 void launch_prologue_batch(const PrologueBeam* recs, int n_beams, long long max_voxels, long long max_lines,
                            int n_sm, int* flags, int* work, cudaStream_t st, int ctas_per_sm);
 void launch_prologue(const float* rho, const GridDev& g, const BeamDev& b, const SettingsDev& s, float* T,
-                     const Inter& inter, int all_voxels, int* aabb, int* list_v, int n_sm, int* flags,
-                     cudaStream_t st, int ctas_per_sm = 8);
+                     const Inter& inter, int all_voxels, int* aabb, bool box, int* list_v, int n_sm, int* flags,
+                     cudaStream_t st, int ctas_per_sm = 8);   // box: the gather needs the TERMA box
 // Frame of the cone directions: off = the room frame (the reference), on =
 // rotated by a beam's world->beam matrix m (row major, xform of ch_beam).
 struct ConeFrame {

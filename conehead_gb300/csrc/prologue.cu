@@ -312,7 +312,8 @@ __device__ __forceinline__ double div_count(float v, double n, double inv_n) {
 // were classified one per warp round, 27 lanes each (a chunk of 32 edge voxels
 // took 32 rounds), and a map's voxels went through those rounds and then again
 // through a per-lane loop with a float64 division per change of value.
-// Measured, whole call: nine MLC beams on 140 x 101 x 112 9425 -> 5060 us, one
+// Measured, whole call: nine MLC beams on 140 x 101 x 112 9425 -> 5060 us with
+// the fixed bound of 0.05 cells, 2660 us with delta and the walk below; one
 // 5 x 5 cm beam on 128^3 227 -> 194 us.
 __device__ __forceinline__ double blocked_fraction(const BeamDev& b, const GridDev& g, int S, const float* pos,
                                                    int& bad) {
@@ -649,26 +650,30 @@ __device__ __forceinline__ void terma_entry(const float* __restrict__ rho, const
       }
     }
   next:
-    // ---- support box of T != 0 (the reference skips T == 0 sources)
-    const bool nz_ = live && Tv != 0.0f;
-    const unsigned m = __ballot_sync(0xffffffffu, nz_);
-    if (m) {
-      int lo0 = nz_ ? x : INT_MAX, hi0 = nz_ ? x : INT_MIN;
-      int lo1 = nz_ ? y : INT_MAX, hi1 = nz_ ? y : INT_MIN;
-      int lo2 = nz_ ? z : INT_MAX, hi2 = nz_ ? z : INT_MIN;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        lo0 = min(lo0, __shfl_xor_sync(0xffffffffu, lo0, o));
-        hi0 = max(hi0, __shfl_xor_sync(0xffffffffu, hi0, o));
-        lo1 = min(lo1, __shfl_xor_sync(0xffffffffu, lo1, o));
-        hi1 = max(hi1, __shfl_xor_sync(0xffffffffu, hi1, o));
-        lo2 = min(lo2, __shfl_xor_sync(0xffffffffu, lo2, o));
-        hi2 = max(hi2, __shfl_xor_sync(0xffffffffu, hi2, o));
-      }
-      if ((threadIdx.x & 31) == 0) {
-        atomicMin(aabb + 0, lo0); atomicMax(aabb + 1, hi0);
-        atomicMin(aabb + 2, lo1); atomicMax(aabb + 3, hi1);
-        atomicMin(aabb + 4, lo2); atomicMax(aabb + 5, hi2);
+    // ---- support box of T != 0 (the reference skips T == 0 sources), for the
+    // gather's tap ranges.  Its six words share one L2 sector, and every chunk
+    // of a beam in flight updated them: those adds took a sixth of the launch
+    // (64 mixed beams, TERMA 3.20 -> 2.69 ms without them; with the walk, the
+    // blocking and the spectrum left out they were three quarters of it).  The
+    // spectral method needs no box, and a chunk inside the box so far adds
+    // nothing.
+    if (aabb) {
+      const bool nz_ = live && Tv != 0.0f;
+      if (__any_sync(0xffffffffu, nz_)) {
+        const int lo0 = __reduce_min_sync(0xffffffffu, nz_ ? x : INT_MAX);
+        const int hi0 = __reduce_max_sync(0xffffffffu, nz_ ? x : INT_MIN);
+        const int lo1 = __reduce_min_sync(0xffffffffu, nz_ ? y : INT_MAX);
+        const int hi1 = __reduce_max_sync(0xffffffffu, nz_ ? y : INT_MIN);
+        const int lo2 = __reduce_min_sync(0xffffffffu, nz_ ? z : INT_MAX);
+        const int hi2 = __reduce_max_sync(0xffffffffu, nz_ ? z : INT_MIN);
+        if ((threadIdx.x & 31) == 0) {
+          if (lo0 < __ldcg(aabb + 0)) atomicMin(aabb + 0, lo0);
+          if (hi0 > __ldcg(aabb + 1)) atomicMax(aabb + 1, hi0);
+          if (lo1 < __ldcg(aabb + 2)) atomicMin(aabb + 2, lo1);
+          if (hi1 > __ldcg(aabb + 3)) atomicMax(aabb + 3, hi1);
+          if (lo2 < __ldcg(aabb + 4)) atomicMin(aabb + 4, lo2);
+          if (hi2 > __ldcg(aabb + 5)) atomicMax(aabb + 5, hi2);
+        }
       }
     }
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(flags, FLAG_PARALLEL_RAY);
@@ -737,7 +742,8 @@ __global__ void __launch_bounds__(256, 3) terma_batch_kernel(const PrologueBeam*
       __syncwarp();
       cur = beam;
     }
-    terma_entry(R.rho, R.g, R.b, R.s, R.T, Inter{}, 0, count, ((c - base) << 5) + lane, R.list_v, R.aabb, flags);
+    terma_entry(R.rho, R.g, R.b, R.s, R.T, Inter{}, 0, count, ((c - base) << 5) + lane, R.list_v,
+                R.box ? R.aabb : nullptr, flags);
   }
 }
 
@@ -963,7 +969,7 @@ void upload_unit_partials() {
 }
 
 void launch_prologue(const float* rho, const GridDev& g, const BeamDev& b, const SettingsDev& s, float* T,
-                     const Inter& inter, int all_voxels, int* aabb, int* list_v, int n_sm, int* flags,
+                     const Inter& inter, int all_voxels, int* aabb, bool box, int* list_v, int n_sm, int* flags,
                      cudaStream_t st, int ctas_per_sm) {
   const long long N = (long long)g.n[0] * g.n[1] * g.n[2];
   const int threads = 256;
@@ -974,7 +980,7 @@ void launch_prologue(const float* rho, const GridDev& g, const BeamDev& b, const
   const long long cap = (long long)n_sm * ctas_per_sm;
   const int grid = (int)(want < cap ? want : cap);
   terma_kernel<<<grid > 0 ? grid : 1, threads, 0, st>>>(rho, g, b, s, T, inter, all_voxels, list_count, list_v,
-                                                        aabb, flags);
+                                                        box ? aabb : nullptr, flags);
 }
 
 // Batched prologue (no intermediates): one cull launch over every beam's grid
