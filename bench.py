@@ -1,7 +1,7 @@
 """Benchmark: beams/s of the collapsed-cone dose engine on GB300.
 
 Workload (one "step"): a batch of --beams beams (default 32: one cull, one
-TERMA and one spectral launch of 16 beam pairs) on the heterogeneous 128^3
+TERMA and one spectral launch group of 32 beams) on the heterogeneous 128^3
 slab phantom (0.25 cm voxels: water, lung slab 0.25 g/cc at depth 5-12 cm,
 bone slab 1.85 g/cc at 14-16 cm, 20 random cuboid inserts of 0.2-2.0
 g/cc), 5 x 5 cm^2 jaw field, gantry uniform in [0, 360), seeded synthetic
@@ -511,39 +511,40 @@ def stage_rooflines(stats, beams, n_vox, cone_bytes, cone_ms, hbm_peak, method):
     return out
 
 
-def spectral_period(n):
-    """FFT period of one axis: the smallest 2^a or 3 * 2^a (a >= 4) >= 2 n - 1."""
-    periods = sorted({16 << a for a in range(9)} | {48 << a for a in range(7)})
-    return next(m for m in periods if m >= 2 * n - 1)
-
-
-# beam pairs per spectral launch (SPEC_MAX_PAIRS of the library)
-SPEC_MAX_PAIRS = 16
-
-
-def spectral_launches(beams, max_pairs=SPEC_MAX_PAIRS):
-    return ((beams + 1) // 2 + max_pairs - 1) // max_pairs
+SPEC_LENGTHS = [16 * k for k in (3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 20, 24, 27, 32)] + \
+    [768, 1024, 1536, 2048, 3072, 4096]
+# beams per spectral launch (SPEC_MAX_BEAMS of the library)
+SPEC_MAX_BEAMS = 32
 
 
 def plane_path(size):
-    """The library's plane path: FFT periods of 256 on every axis (grids of
-    97-128 voxels per axis): z forward, one fused plane kernel (y and x
-    transforms, the S^ product and their inverses on chip), z inverse."""
-    return all(spectral_period(int(k)) == 256 for k in size)
+    """The library's plane path (97-128 voxels along x and y): z forward, one
+    fused plane kernel (y and x transforms, the S^ product and their inverses
+    on chip), z inverse."""
+    return all(96 < int(k) <= 128 for k in size[:2])
 
 
-def spectral_bytes(size, beams, max_pairs=SPEC_MAX_PAIRS):
+def spectral_lengths(size):
+    """Transform lengths: >= 2 n - 1 along x and y, >= n along z."""
+    M = [next(m for m in SPEC_LENGTHS if m >= need) for need in (2 * size[0] - 1, 2 * size[1] - 1, size[2])]
+    return [256, 256, M[2]] if plane_path(size) else M
+
+
+def spectral_launches(beams, max_beams=SPEC_MAX_BEAMS):
+    return (beams + max_beams - 1) // max_beams
+
+
+def spectral_bytes(size, beams, max_beams=SPEC_MAX_BEAMS):
     """HBM bytes the FFT passes must move for `beams` beams of one grid: per
-    pair of beams the two TERMA volumes in and two doses out (16 N), the
-    intermediate A [nx][ny][Mz] (complex float32) written and read twice,
-    B [nx][My][Mz] likewise on the five-pass path (the plane path keeps it on
-    chip), and S^ [Mx][My][Mz] read once per launch."""
+    beam the TERMA volume in and the dose out (8 N), the intermediate
+    A [nx][ny][Mz] (complex float32) written and read twice, B [nx][My][Mz]
+    likewise on the five-pass path (the plane path keeps it on chip), and
+    S^ [Mx][My][Mz] read once per launch."""
     nx, ny, nz = (int(k) for k in size)
-    Mx, My, Mz = (spectral_period(k) for k in (nx, ny, nz))
-    pairs = (beams + 1) // 2
+    Mx, My, Mz = spectral_lengths((nx, ny, nz))
     a = nx * ny * Mz * 8
     b = 0 if plane_path(size) else nx * My * Mz * 8
-    return pairs * (16 * nx * ny * nz + 4 * a + 4 * b) + spectral_launches(beams, max_pairs) * Mx * My * Mz * 8
+    return beams * (8 * nx * ny * nz + 4 * a + 4 * b) + spectral_launches(beams, max_beams) * Mx * My * Mz * 8
 
 
 def config(args, beams_per_step=None):
@@ -854,9 +855,9 @@ def run_ours(args):
                          "traffic_over_algorithmic": traffic / alg_bytes if traffic else None,
                          "pass_bytes_per_step": pass_bytes,
                          "pass_traffic_frac": pass_bytes / (cone_ms * 1e-3) / 1e9 / hbm_peak,
-                         "pass_basis": ("bytes the FFT pass structure must move (TERMA pair in, the A "
+                         "pass_basis": ("bytes the FFT pass structure must move (TERMA in, the A "
                                         "intermediate (and B on the five-pass path) written and read twice, "
-                                        "dose pair out, S^ once per launch) over the stage time: how well the "
+                                        "dose out, S^ once per launch) over the stage time: how well the "
                                         "passes stream, not how close the stage is to its bound")
                                        if method == "spectral" else
                                        "as achieved",

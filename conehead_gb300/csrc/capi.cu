@@ -515,17 +515,29 @@ SpecGrid spec_grid(const ch_plan* P, const int* n, const int* M, int zp, int con
     g.logL[k] = k == 2 ? spec_lines_log2(M[2]) : spec_pass_lines_log2(M[k], M[2]);
     g.tw[k] = P->spec_tw.as<float2>() + spec_twiddle_offset(M[k]);
   }
+  g.tq = g.tw[2] + M[2];
   g.zp = zp;
   g.conj = conj;
   g.shat = shat;
-  g.plane = spec_plane_path(M) && n[0] <= SPEC_PLANE_M / 2 && n[1] <= SPEC_PLANE_M / 2 && n[2] <= SPEC_PLANE_M / 2;
+  g.plane = spec_plane_path(M) ? 1 : 0;
   g.lp = g.plane ? spec_plane_pitch(n) : 0;
   return g;
 }
 
+// The lengths of a grid's transforms (0: none).
+void spec_lengths_of(const int* n, int* M) {
+  M[0] = spec_period(n[0]);
+  M[1] = spec_period(n[1]);
+  M[2] = spec_length_z(n[2]);
+  // 97-128 voxels on both: the plane path, also where 240 would hold 2 n - 1
+  if (n[0] > 96 && n[0] <= 128 && n[1] > 96 && n[1] <= 128) M[0] = M[1] = SPEC_PLANE_M;
+}
+
 // S^ of grid shape n for stencil set S: the current tap weights summed per
 // offset o with |o_k| <= n_k - 1 (float64 sums in offset order, times
-// 1/(Mx My Mz)), placed at o mod M, then three forward FFT passes.  Cached
+// 1/(Mx My Mz)), placed at o mod M along x and y; along z modulo (z^Mz + i),
+// i.e. o_z >= 0 at o_z and o_z < 0 at Mz + o_z in the imaginary part
+// (z^o = -z^(2 Mz + o) = -z^Mz z^(Mz + o) = i z^(Mz + o)); then three forward FFT passes.  Cached
 // per (set, shape), least recently used out past kSpecEntries while no
 // captured batch holds one.
 constexpr size_t kSpecEntries = 8;
@@ -549,7 +561,8 @@ ch_status spec_shat(ch_plan* P, const StencilSet& S, const int* n, cudaStream_t 
                                 });
     P->spec.erase(lru);
   }
-  const int M[3] = {spec_period(n[0]), spec_period(n[1]), spec_period(n[2])};
+  int M[3];
+  spec_lengths_of(n, M);
   const size_t vol = (size_t)M[0] * M[1] * M[2];
   std::vector<int4> taps(S.total_taps);
   std::vector<short4> offs(S.total_taps);
@@ -561,7 +574,9 @@ ch_status spec_shat(ch_plan* P, const StencilSet& S, const int* n, cudaStream_t 
   for (size_t t = 0; t < taps.size(); ++t) {
     const short4 o = offs[t];
     if (std::abs((int)o.x) > n[0] - 1 || std::abs((int)o.y) > n[1] - 1 || std::abs((int)o.z) > n[2] - 1) continue;
-    const long long i = (((long long)(o.x + M[0]) % M[0]) * M[1] + (o.y + M[1]) % M[1]) * M[2] + (o.z + M[2]) % M[2];
+    // float index: the real part for o_z >= 0, the imaginary part below
+    const long long i = 2 * ((((long long)(o.x + M[0]) % M[0]) * M[1] + (o.y + M[1]) % M[1]) * M[2] +
+                             (o.z < 0 ? M[2] + o.z : o.z)) + (o.z < 0 ? 1 : 0);
     float w;
     std::memcpy(&w, &taps[t].w, 4);
     ent.emplace_back(i, w);
@@ -582,32 +597,27 @@ ch_status spec_shat(ch_plan* P, const StencilSet& S, const int* n, cudaStream_t 
   std::unique_ptr<SpecEntry> E(new SpecEntry());
   E->set = &S;
   for (int k = 0; k < 3; ++k) E->n[k] = n[k];
-  DevBuf d_idx, d_val, s_real, work;
+  DevBuf d_idx, d_val, work;
   auto cleanup = [&]() {
     d_idx.release();
     d_val.release();
-    s_real.release();
     work.release();
   };
+  const bool plane = spec_plane_path(M);
   cudaError_t e = E->shat.ensure(vol * sizeof(float2));
-  if (e == cudaSuccess) e = s_real.ensure(vol * sizeof(float));
-  if (e == cudaSuccess) e = work.ensure(vol * sizeof(float2));
+  if (e == cudaSuccess && plane) e = work.ensure(vol * sizeof(float2));
   if (e == cudaSuccess) e = d_idx.ensure(std::max<size_t>(idx.size(), 1) * sizeof(long long));
   if (e == cudaSuccess) e = d_val.ensure(std::max<size_t>(val.size(), 1) * sizeof(float));
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_idx.p, idx.data(), idx.size() * sizeof(long long), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_val.p, val.data(), val.size() * sizeof(float), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(s_real.p, 0, vol * sizeof(float), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(E->shat.p, 0, vol * sizeof(float2), s);
   if (e != cudaSuccess) {
     cleanup();
     return fail(CH_ERR_DEVICE, std::string("spectral stencil: ") + cudaGetErrorString(e));
   }
-  SpecLaunch L{};
-  L.g = spec_grid(P, M, M, M[2], 0, nullptr);
-  L.n_pairs = 1;
-  L.p[0] = SpecPair{s_real.as<float>(), nullptr, nullptr, nullptr, work.as<float2>(), E->shat.as<float2>(),
-                    nullptr, nullptr};
-  launch_spec_build(L, d_idx.as<long long>(), d_val.as<float>(), (int)idx.size(), s_real.as<float>(), s);
-  if (spec_plane_path(M)) {
+  launch_spec_build(spec_grid(P, M, M, M[2], 0, nullptr), d_idx.as<long long>(), d_val.as<float>(), (int)idx.size(),
+                    E->shat.as<float2>(), s);
+  if (plane) {
     // the plane path reads S^ plane by plane: [Mz][My][Mx], transposed into
     // the work buffer, which then becomes the cached S^ (the untransposed
     // copy is released with the other build buffers)
@@ -903,17 +913,17 @@ ch_status stage_records(ch_plan* P, const std::vector<Seg>& segs, cudaStream_t s
 }
 
 // ------------------------------------------------- spectral cone layout --
-// Beams of one grid shape are paired in call order; a launch takes up to
-// SPEC_MAX_PAIRS pairs of one shape, and the launches of a batch run one
-// after another in one work arena (A and B of each pair of the launch).
-struct SpecPlanPair {
-  int j1, j2;                // beams (j2 = -1: the first alone)
+// Beams of one grid shape share a launch of up to SPEC_MAX_BEAMS, in call
+// order; the launches of a batch run one after another in one work arena (A and
+// B of each beam of the launch).
+struct SpecPlanBeam {
+  int job;
   size_t a_off, b_off;       // float2 offsets in the work arena
 };
 struct SpecPlanLaunch {
   int n[3], M[3];
   const float2* shat = nullptr;
-  std::vector<SpecPlanPair> pairs;
+  std::vector<SpecPlanBeam> beams;
 };
 struct SpecLayout {
   std::vector<SpecPlanLaunch> launches;
@@ -923,11 +933,12 @@ struct SpecLayout {
 constexpr long long kSpecMaxVolume = 1ll << 28;   // largest Mx My Mz (S^ of 2 GiB)
 
 bool spec_fits(const int* n) {
+  int M[3];
+  spec_lengths_of(n, M);
   long long v = 1;
   for (int k = 0; k < 3; ++k) {
-    const int m = spec_period(n[k]);
-    if (m == 0) return false;
-    v *= m;
+    if (M[k] == 0) return false;
+    v *= M[k];
   }
   return v <= kSpecMaxVolume;
 }
@@ -945,28 +956,27 @@ SpecLayout spec_layout(int n, const ch_grid* grids) {
         done[j] = 1;
       }
     const int* d = grids[i].n;
-    const int M[3] = {spec_period(d[0]), spec_period(d[1]), spec_period(d[2])};
+    int M[3];
+    spec_lengths_of(d, M);
     // the plane path keeps A plane-major (pitch spec_plane_pitch) and needs no B
     const bool plane = spec_plane_path(M);
     const size_t a_sz = plane ? (size_t)M[2] * spec_plane_pitch(d) : (size_t)d[0] * d[1] * M[2];
     const size_t b_sz = plane ? 0 : (size_t)d[0] * M[1] * M[2];
-    for (size_t p = 0; p < group.size(); p += 2 * SPEC_MAX_PAIRS) {
+    for (size_t p = 0; p < group.size(); p += SPEC_MAX_BEAMS) {
       SpecPlanLaunch l;
       for (int k = 0; k < 3; ++k) {
         l.n[k] = d[k];
         l.M[k] = M[k];
       }
       size_t off = 0;
-      const size_t end = std::min(group.size(), p + 2 * SPEC_MAX_PAIRS);
-      for (size_t q = p; q < end; q += 2) {
-        SpecPlanPair pr;
-        pr.j1 = group[q];
-        pr.j2 = q + 1 < end ? group[q + 1] : -1;
-        pr.a_off = off;
+      for (size_t q = p; q < std::min(group.size(), p + SPEC_MAX_BEAMS); ++q) {
+        SpecPlanBeam b;
+        b.job = group[q];
+        b.a_off = off;
         off += (a_sz + 31) / 32 * 32;
-        pr.b_off = off;
+        b.b_off = off;
         off += (b_sz + 31) / 32 * 32;
-        l.pairs.push_back(pr);
+        l.beams.push_back(b);
       }
       L.arena = std::max(L.arena, off);
       L.launches.push_back(std::move(l));
@@ -1251,21 +1261,16 @@ ch_status enqueue_batch(ch_plan* P, const BatchPlan& B, const Scratch& S, const 
     if (ev) CH_CUDA(cudaEventRecord(ev[2], s));
     for (const SpecPlanLaunch& l : B.spec.launches) {
       SpecLaunch L{};
-      const BeamJob& J0 = B.jobs[l.pairs[0].j1];
-      L.g = spec_grid(P, l.n, l.M, J0.g.zp, 0, l.shat);
-      L.n_pairs = (int)l.pairs.size();
-      for (int q = 0; q < L.n_pairs; ++q) {
-        const SpecPlanPair& pr = l.pairs[q];
-        const BeamJob& J1 = B.jobs[pr.j1];
-        const BeamJob* J2 = pr.j2 >= 0 ? &B.jobs[pr.j2] : nullptr;
+      L.g = spec_grid(P, l.n, l.M, B.jobs[l.beams[0].job].g.zp, 0, l.shat);
+      L.n_beams = (int)l.beams.size();
+      for (int q = 0; q < L.n_beams; ++q) {
+        const SpecPlanBeam& b = l.beams[q];
+        const BeamJob& J = B.jobs[b.job];
         // line flags exist when the batched prologue ran (no intermediates)
-        const unsigned char* f1 = inter ? nullptr : reinterpret_cast<const unsigned char*>(S.list_v + J1.f_off);
-        const unsigned char* f2 =
-            (inter || !J2) ? nullptr : reinterpret_cast<const unsigned char*>(S.list_v + J2->f_off);
-        L.p[q] = SpecPair{S.T + J1.t_off, J2 ? S.T + J2->t_off : nullptr, f1, f2, S.spec + pr.a_off,
-                          S.spec + pr.b_off, J1.dose, J2 ? J2->dose : nullptr};
+        const unsigned char* flags_l = inter ? nullptr : reinterpret_cast<const unsigned char*>(S.list_v + J.f_off);
+        L.p[q] = SpecBeam{S.T + J.t_off, flags_l, S.spec + b.a_off, S.spec + b.b_off, J.dose};
       }
-      launch_spec_pairs(L, s);
+      launch_spec_beams(L, s);
       CH_CUDA(cudaGetLastError());
     }
     if (ev) CH_CUDA(cudaEventRecord(ev[3], s));
@@ -1690,11 +1695,10 @@ ch_status cone_operator(ch_plan* P, const ch_grid& grid, const float* in_dense, 
     const SpecPlanLaunch& l = L.launches[0];
     SpecLaunch SL{};
     SL.g = spec_grid(P, l.n, l.M, grid.n[2], transpose ? 1 : 0, shat);
-    SL.n_pairs = 1;
+    SL.n_beams = 1;
     float2* w = P->spec_work.as<float2>();
-    SL.p[0] = SpecPair{in_dense, nullptr, nullptr, nullptr, w + l.pairs[0].a_off, w + l.pairs[0].b_off, out,
-                       nullptr};
-    launch_spec_pairs(SL, s);
+    SL.p[0] = SpecBeam{in_dense, nullptr, w + l.beams[0].a_off, w + l.beams[0].b_off, out};
+    launch_spec_beams(SL, s);
     CH_CUDA(cudaGetLastError());
     return CH_OK;
   }

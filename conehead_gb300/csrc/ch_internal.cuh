@@ -238,65 +238,70 @@ struct Inter {
 };
 
 // ---------------------------------------------------- spectral cone stage --
-// The cone stage as one circular convolution per grid shape (spectral.cu):
-// periods M_k = the smallest 2^a or 3 * 2^a >= 2 n_k - 1 (at least
-// SPEC_MIN_PERIOD), pairs of beams per complex transform.
-constexpr int SPEC_THREADS = 256;
-constexpr int SPEC_CTAS_PER_SM = 3;       // register budget of the passes (85 per thread)
+// The cone stage as one convolution per grid shape (spectral.cu): periods
+// M_k = the smallest allowed length >= 2 n_k - 1 along x and y, M_z = the
+// smallest >= nz along z (spec_lengths), one transform per beam.
+constexpr int SPEC_THREADS = 256;         // general kernels
+constexpr int SPEC_CTAS_PER_SM = 3;       // their register budget (85 per thread)
 constexpr int SPEC_ELEMS = 4096;          // complex values per CTA: 4096 / M lines of period M
-constexpr int SPEC_MIN_PERIOD = 16, SPEC_MAX_PERIOD = 4096;
-constexpr int SPEC_MAX_PAIRS = 16;        // beam pairs per launch (their work buffers coexist)
+constexpr int SPEC_MIN_GENERAL = 768, SPEC_MAX_PERIOD = 4096;
+constexpr int SPEC_MAX_BEAMS = 32;        // beams per launch (their work buffers coexist)
 constexpr int SPEC_SMEM = 2 * SPEC_ELEMS * 8;   // two ping-pong buffers of float2 per CTA
-struct SpecPair {
-  const float* t1;   // TERMA of the first beam [nx][ny][zp]
-  const float* t2;   // of the second (NULL: none)
-  const unsigned char* l1;  // lines of t1 that may be nonzero (NULL: every line is read)
-  const unsigned char* l2;  // of t2
-  float2* a;         // [nx][ny][Mz]
-  float2* b;         // [nx][My][Mz]
-  float* d1;         // dose of the first beam [nx][ny][nz]
-  float* d2;         // of the second (NULL: none)
+struct SpecBeam {
+  const float* t;          // TERMA [nx][ny][zp]
+  const unsigned char* l;  // lines of t that may be nonzero (NULL: every line is read)
+  float2* a;               // [nx][ny][Mz]
+  float2* b;               // [nx][My][Mz]
+  float* d;                // dose [nx][ny][nz]
 };
 struct SpecGrid {
   int n[3], M[3];
-  int logL[3];             // log2 of the lines per CTA of the pass along x, y, z
+  int logL[3];             // log2 of the lines per CTA of the general pass along x, y, z
   int zp;                  // z pitch of the TERMA volumes
   int conj;                // multiply by conj(S^): the transposed cone
   const float2* tw[3];     // twiddles exp(-2 pi i k / M_axis)
+  const float2* tq;        // quarter steps exp(-2 pi i k / (4 Mz)): the twist along z
   const float2* shat;      // S^ [Mx][My][Mz], 1/(Mx My Mz) folded in; [Mz][My][Mx] on the plane path
   int plane;               // the plane path (spec_plane_path): A = [Mz][lp] plane-major, no B
   int lp;                  // plane pitch of A on the plane path (nx ny rounded up to 32)
 };
 struct SpecLaunch {
   SpecGrid g;
-  int n_pairs;
-  SpecPair p[SPEC_MAX_PAIRS];
+  int n_beams;
+  SpecBeam p[SPEC_MAX_BEAMS];
 };
-int spec_period(int n);                  // 0 when no period up to SPEC_MAX_PERIOD holds 2n - 1
+// forward transform of full lines in place: element i of line (o, c), c < 16,
+// at data + (o / nb) os1 + (o mod nb) os2 + c cs + i is
+struct SpecFull {
+  float2* data;
+  const float2* tw;
+  const float2* tq;        // multiplied in first (NULL: not)
+  int nb;
+  size_t os1, os2, cs, is;
+};
+int spec_period(int n);                  // 0 when no length up to SPEC_MAX_PERIOD holds 2n - 1
+int spec_length_z(int nz);               // 0 when none holds nz
 int spec_lines_log2(int M);
 int spec_pass_lines_log2(int M, int Mz);
-std::vector<float2> spec_twiddles();      // every period (ascending), back to back
-size_t spec_twiddle_offset(int M);
-cudaError_t setup_spec_kernels();        // allow SPEC_SMEM of dynamic shared memory
-void launch_spec_pairs(const SpecLaunch& L, cudaStream_t st);
-// The plane path: periods of 256 on every axis (grids of 97 to 128 voxels
-// per axis).  z forward into plane-major A[kz][x y], one cluster of two CTAs
-// per (pair, kz) plane for the y and x transforms, the S^ product and their
-// inverses (the plane's spectrum held in the pair's shared memory), z
-// inverse from A.  S^ is then kept as [Mz][My][Mx].
+std::vector<float2> spec_twiddles();      // every length (ascending), back to back
+size_t spec_twiddle_offset(int M);       // of exp(-2 pi i k / M); the quarter steps follow
+cudaError_t setup_spec_kernels();        // allow the kernels their dynamic shared memory
+void launch_spec_beams(const SpecLaunch& L, cudaStream_t st);
+// The plane path: periods of 256 along x and y (97 to 128 voxels).  z forward
+// into plane-major A[kz][x y], one cluster of two CTAs per (beam, kz) plane for
+// the y and x transforms, the S^ product and their inverses (the plane's
+// spectrum held in the pair's shared memory), z inverse from A.  S^ is then
+// kept as [Mz][My][Mx].
 constexpr int SPEC_PLANE_M = 256;
 // half the plane spectrum, an exchange buffer per warp, the twiddle table
 constexpr int SPEC_PLANE_SMEM = (128 * 128 + 16 * 2 * 256 + 16 * 18) * 8;
-inline bool spec_plane_path(const int* M) {
-  return M[0] == SPEC_PLANE_M && M[1] == SPEC_PLANE_M && M[2] == SPEC_PLANE_M;
-}
+inline bool spec_plane_path(const int* M) { return M[0] == SPEC_PLANE_M && M[1] == SPEC_PLANE_M; }
 inline int spec_plane_pitch(const int* n) { return (n[0] * n[1] + 31) / 32 * 32; }
 // S^ [Mx][My][Mz] -> [Mz][My][Mx]
 void launch_spec_transpose(const float2* in, float2* out, int Mx, int My, int Mz, cudaStream_t st);
-// S^ of one grid shape: scatter the stencil values into the real volume
-// s_real (zeroed, [Mx][My][Mz] = L.p[0].t1), then three forward passes
-// (L.g.n = M, L.p[0].a = work, L.p[0].b = S^)
-void launch_spec_build(const SpecLaunch& L, const long long* idx, const float* val, int n_val, float* s_real,
+// S^ of one grid shape, in place: scatter the folded stencil's values (float
+// indexes into s, zeroed, [Mx][My][Mz]), then three forward passes
+void launch_spec_build(const SpecGrid& g, const long long* idx, const float* val, int n_val, float2* s,
                        cudaStream_t st);
 
 // One beam of a batched prologue (device record).

@@ -1,0 +1,26 @@
+// FFT passes of lengths 16 N2 with a 16-point and an N2-point DFT in
+// registers and one shared-memory exchange between them (spectral.cu has the
+// method; spectral_z.cu, spectral_y.cu and spectral_x.cu the kernels).
+//
+// Lengths: N2 in SPEC_N2, i.e. 48 to 512.  2^a and 3 * 2^a alone wasted up to
+// half of an axis: 160 voxels need a period of 319 and took 384 (x pass of 16
+// beams 1515 us, 913 us at 320), 201 need 401 and took 512 through four
+// shared-memory stages of the general kernels (x pass of one beam 871 us at two
+// beams' cost, 236 us at 432).
+#pragma once
+
+#include "spectral_dft.cuh"
+
+namespace ch {
+
+#define SPEC_N2(X) X(3) X(4) X(5) X(6) X(8) X(9) X(10) X(12) X(15) X(16) X(18) X(20) X(24) X(27) X(32)
+
+// A CTA takes 16 lines: 16 N2 threads in the 16-point stages, 256 in the
+// N2-point ones.  CTAs per SM by registers (the N2-point stage holds 4 N2
+// values) and, along x, by shared memory.
+template <int N2>
+constexpr int r16n_threads() { return 16 * N2 > 256 ? 16 * N2 : 256; }
+template <int N2>
+constexpr int r16n_ctas() { return N2 <= 12 ? 4 : N2 <= 16 ? 3 : N2 <= 24 ? 2 : 1; }
+
+}  // namespace ch
