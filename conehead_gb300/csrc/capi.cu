@@ -128,6 +128,8 @@ struct ch_plan {
   int live_batches = 0;      // captured batches reading this plan's stencils
   long long wait_limit = 0;  // gather pipeline waits (try_wait iterations); 0 = MBAR_LIMIT
   int withhold = 0;          // test hook of the expired-wait path (ch_plan_set_wait_limit)
+  int epoch = 0;             // of the last call with the one-launch prologue
+  bool flags_by_epoch = false;   // the last call reports failures in counters[6] == epoch, not in counters[1]
   int reweights = 0;         // spectrum switches served by reweighting the stencils
   std::vector<std::unique_ptr<FrameStencils>> frames;   // beam-frame cone stencils by orientation
   uint64_t use_clock = 0;
@@ -1221,6 +1223,52 @@ Inter make_inter(const ch_intermediates* inter, int& all) {
   return in;
 }
 
+// The spectral cone stage of a batch: launch after launch in the work arena;
+// every dose voxel is written.  all_lines: no line flags exist (the prologue
+// wrote intermediates), every TERMA line is read.
+ch_status enqueue_spectral(ch_plan* P, const BatchPlan& B, const Scratch& S, bool all_lines, const cudaEvent_t* ev,
+                           cudaStream_t s) {
+  if (ev) CH_CUDA(cudaEventRecord(ev[2], s));
+  for (const SpecPlanLaunch& l : B.spec.launches) {
+    SpecLaunch L{};
+    L.g = spec_grid(P, l.n, l.M, B.jobs[l.beams[0].job].g.zp, 0, l.shat);
+    L.n_beams = (int)l.beams.size();
+    for (int q = 0; q < L.n_beams; ++q) {
+      const SpecPlanBeam& b = l.beams[q];
+      const BeamJob& J = B.jobs[b.job];
+      const unsigned char* lines = all_lines ? nullptr : reinterpret_cast<const unsigned char*>(S.list_v + J.f_off);
+      L.p[q] = SpecBeam{S.T + J.t_off, lines, S.spec + b.a_off, S.spec + b.b_off, J.dose};
+    }
+    launch_spec_beams(L, s);
+    CH_CUDA(cudaGetLastError());
+  }
+  if (ev) CH_CUDA(cudaEventRecord(ev[3], s));
+  return CH_OK;
+}
+
+// Whether a batch takes the one-launch prologue: a few small beams, at most
+// FUSED_MAX_LINES (x, y) lines in all and, by the opening times the grid's
+// length along the beam, FUSED_MAX_CHUNKS chunks of 32 voxels in the field.
+// Measured, whole calls with a turned collimator, two launches and a copy
+// against one: 64^3 12 x 12 cm 98.7 / 89.8 us, 4 beams 5 x 5 cm on 64^3
+// (16384 lines) 121 / 117, 96^3 8 x 8 cm (9216) 109.5 / 111.2, 128^3 5 x 5 cm
+// (16384) 134.7 / 133.4, 7 x 7 cm 146 / 160, 150 x 130 lines 217 / 230: a warp
+// per line costs more than the cull once lines outnumber the resident warps.
+constexpr int FUSED_MAX_LINES = 8192, FUSED_MAX_CHUNKS = 6000;
+bool fused_prologue(const BatchPlan& B) {
+  if (B.jobs.size() > FUSED_MAX_BEAMS) return false;
+  double vox = 0.0;
+  long long lines = 0;
+  for (const BeamJob& J : B.jobs) {
+    const float* sp = J.g.spacing;
+    const double len = std::max(J.g.n[0] * (double)sp[0], J.g.n[1] * (double)sp[1]);
+    const double area = std::max(0.0f, J.b.cx_hi - J.b.cx_lo) * (double)std::max(0.0f, J.b.cz_hi - J.b.cz_lo);
+    vox += std::min((double)J.g.n[0] * J.g.n[1] * J.g.n[2], area * len / ((double)sp[0] * sp[1] * sp[2]));
+    lines += (long long)J.g.n[0] * J.g.n[1];
+  }
+  return lines <= FUSED_MAX_LINES && vox <= 32.0 * FUSED_MAX_CHUNKS;
+}
+
 // The device work of a batch (records already on the device): reset,
 // prologues, dose zeroing, tap ranges, one persistent gather.  Only kernel
 // launches and memsets, so it can be captured into a CUDA graph.  ev (4
@@ -1255,27 +1303,7 @@ ch_status enqueue_batch(ch_plan* P, const BatchPlan& B, const Scratch& S, const 
     CH_CUDA(cudaGetLastError());
   }
   if (ev) CH_CUDA(cudaEventRecord(ev[1], s));
-  if (B.spectral) {
-    // FFT convolution, launch after launch in the work arena; every dose
-    // voxel is written
-    if (ev) CH_CUDA(cudaEventRecord(ev[2], s));
-    for (const SpecPlanLaunch& l : B.spec.launches) {
-      SpecLaunch L{};
-      L.g = spec_grid(P, l.n, l.M, B.jobs[l.beams[0].job].g.zp, 0, l.shat);
-      L.n_beams = (int)l.beams.size();
-      for (int q = 0; q < L.n_beams; ++q) {
-        const SpecPlanBeam& b = l.beams[q];
-        const BeamJob& J = B.jobs[b.job];
-        // line flags exist when the batched prologue ran (no intermediates)
-        const unsigned char* flags_l = inter ? nullptr : reinterpret_cast<const unsigned char*>(S.list_v + J.f_off);
-        L.p[q] = SpecBeam{S.T + J.t_off, flags_l, S.spec + b.a_off, S.spec + b.b_off, J.dose};
-      }
-      launch_spec_beams(L, s);
-      CH_CUDA(cudaGetLastError());
-    }
-    if (ev) CH_CUDA(cudaEventRecord(ev[3], s));
-    return CH_OK;
-  }
+  if (B.spectral) return enqueue_spectral(P, B, S, inter != nullptr, ev, s);
   for (int i = 0; i < n; ++i)
     CH_CUDA(cudaMemsetAsync(B.jobs[i].dose, 0, (size_t)B.jobs[i].g.n[0] * B.jobs[i].g.n[1] * B.jobs[i].g.n[2] * 4,
                             s));
@@ -1297,7 +1325,9 @@ ch_status run_group(ch_plan* P, int n, const ch_grid* grids, const float* const*
   ch_status st = plan_batch(P, n, grids, rho, swap_xy, beams, settings, dose, s, B, set);
   if (st != CH_OK) return st;
   const ScratchNeed need = scratch_need(n, grids, B.U, B.spectral && !scatter);
+  const bool new_counters = P->counters.bytes == 0;
   for (int k = 0; k < N_SCRATCH; ++k) CH_CUDA(const_cast<DevBuf*>(scratch_bufs(P, k))->ensure(need.bytes[k]));
+  if (new_counters) CH_CUDA(cudaMemsetAsync(P->counters.p, 0, need.bytes[2], s));
   const Scratch S{P->T.as<float>(),          P->aabb.as<int>(),           P->counters.as<int>(),
                   P->ranges.as<uint32_t>(),  P->cranges.as<uint32_t>(),   P->cone_beams.as<ConeBeam>(),
                   P->range_beams.as<RangeBeam>(), P->list_v.as<int>(),    P->spec_work.as<float2>(),
@@ -1308,6 +1338,21 @@ ch_status run_group(ch_plan* P, int n, const ch_grid* grids, const float* const*
   P->stats.n_unique_dirs = B.U;
   P->stats_pending = true;
   P->last_stream = s;
+  P->flags_by_epoch = false;
+  if (B.spectral && !scatter && !inter && fused_prologue(B)) {
+    P->epoch += 1;
+    P->flags_by_epoch = true;
+    const std::vector<PrologueBeam> pb = make_prologue_records(B, S);
+    FusedRecords rec;
+    std::memcpy(rec.r, pb.data(), pb.size() * sizeof(PrologueBeam));
+    long long max_lines = 1;
+    for (const BeamJob& J : B.jobs) max_lines = std::max(max_lines, (long long)J.g.n[0] * J.g.n[1]);
+    CH_CUDA(cudaEventRecord(P->ev[0], s));
+    launch_prologue_fused(rec, n, max_lines, S.counters + 6, P->epoch, s);
+    CH_CUDA(cudaGetLastError());
+    CH_CUDA(cudaEventRecord(P->ev[1], s));
+    return enqueue_spectral(P, B, S, false, P->ev, s);
+  }
   if (scatter) {
     // plain path: prologues, then one per-voxel scatter launch per beam
     int* flags = S.counters + 1;
@@ -1610,6 +1655,7 @@ ch_status ch_dose_static(ch_plan* P, const ch_grid* grid, const float* rho, int 
   // rather than an earlier call's timings
   P->stats_pending = false;
   P->stats = ch_stats{};
+  P->flags_by_epoch = false;
   // aabb and the list count must start from their reset values; TERMA is
   // rewritten in full by the prologue and the range tables by range_kernel
   launch_init_scratch(aabb, 1, counters, s);
@@ -1794,6 +1840,7 @@ ch_status ch_cone(ch_plan* P, const ch_grid* grid, const float* in, float* out, 
   if ((st = ensure_stencils(P, grid->spacing, grid->n, s)) != CH_OK) return st;
   CH_CUDA(P->aabb.ensure(8 * sizeof(int)));
   CH_CUDA(P->counters.ensure(8 * sizeof(int)));
+  P->flags_by_epoch = false;
   launch_init_scratch(P->aabb.as<int>(), 1, P->counters.as<int>(), s);
   st = cone_operator(P, *grid, in, out, transpose != 0, P->aabb.as<int>(), nullptr, s);
   if (st != CH_OK) return st;
@@ -1844,6 +1891,7 @@ ch_status ch_dose_adjoint(ch_plan* P, const ch_grid* grid, const float* rho, int
   int* flags = counters + 1;
   const BeamDev b = make_beam(*beam, *grid, settings->samples);
   const SettingsDev sd = make_settings(*settings);
+  P->flags_by_epoch = false;
   launch_init_scratch(box, 2, counters, s);
   // forward prologue: TERMA, its box and the list of voxels the beam reaches
   launch_prologue(rho, g, b, sd, P->T.as<float>(), Inter{}, 0, box, !spec_batch(P, 1, grid), P->list_v.as<int>(),
@@ -2116,9 +2164,9 @@ ch_status ch_plan_sync(ch_plan* P, void* stream) {
   CH_CUDA(cudaSetDevice(P->device));
   CH_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
   if (!P->counters.p) return CH_OK;
-  int c[4];
+  int c[8];
   CH_CUDA(cudaMemcpy(c, P->counters.p, sizeof(c), cudaMemcpyDeviceToHost));
-  const int flags = c[1];
+  const int flags = P->flags_by_epoch ? (c[6] == P->epoch ? FLAG_PARALLEL_RAY : 0) : c[1];
   if (flags & FLAG_TIMEOUT) return fail(CH_ERR_TIMEOUT, "a bounded device wait expired in the cone stage");
   if (flags & FLAG_PARALLEL_RAY) return fail(CH_ERR_PARALLEL_RAY, "no intersection or line is within plane");
   return CH_OK;

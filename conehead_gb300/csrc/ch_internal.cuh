@@ -319,7 +319,16 @@ struct PrologueBeam {
   int box;           // 1: the gather needs the TERMA box
 };
 
+// Records of the one-launch prologue, passed as a kernel parameter.
+constexpr int FUSED_MAX_BEAMS = 4;
+struct FusedRecords {
+  PrologueBeam r[FUSED_MAX_BEAMS];
+};
+static_assert(sizeof(FusedRecords) <= 3968, "the records fit the smallest kernel parameter space");
+
 // ------------------------------------------------------------ launchers --
+void launch_prologue_fused(const FusedRecords& recs, int n_beams, long long max_lines, int* flag_word, int epoch,
+                           cudaStream_t st);
 void upload_unit_partials();
 // work: a zeroed int, the TERMA launch's chunk counter
 void launch_prologue_batch(const PrologueBeam* recs, int n_beams, long long max_voxels, long long max_lines,

@@ -463,6 +463,26 @@ __device__ __forceinline__ bool line_outside(const GridDev& g, const BeamDev& b,
   return xhi < b.cx_lo - M || xlo > b.cx_hi + M || zhi < b.cz_lo - M || zlo > b.cz_hi + M;
 }
 
+// Whether the beam may reach the voxel centred at pos: its projection against
+// the opening widened by the sub-samples' margin.
+__device__ __forceinline__ bool cull_candidate(const BeamDev& b, const float* pos) {
+  if (!b.cull_enable) return true;
+  const float np_ = b.vyf[0] * pos[0] + b.vyf[1] * pos[1] + b.vyf[2] * pos[2];
+  const float m0p = b.m0f[0] * pos[0] + b.m0f[1] * pos[1] + b.m0f[2] * pos[2];
+  const float m2p = b.m2f[0] * pos[0] + b.m2f[1] * pos[1] + b.m2f[2] * pos[2];
+  const float depth = np_ - b.a_nS;   // -n . (S - p)
+  if (!(depth > 0.2f * fabsf(b.a_K))) return true;
+  // one fast reciprocal: its ~2 ulp error is far inside the 0.01 cm
+  // margin, so the candidate set stays a superset of the beam
+  const float inv_depth = __fdividef(1.0f, depth);
+  const float si = -b.a_K * inv_depth;
+  const float xb = b.a_c0 + si * (b.a_m0S - m0p);
+  const float zb = b.a_c2 + si * (b.a_m2S - m2p);
+  const float lat = fmaxf(fabsf(b.a_m0S - m0p), fabsf(b.a_m2S - m2p)) * inv_depth;
+  const float margin = b.cull_margin_k * fabsf(b.a_K) * inv_depth * (1.0f + lat) + 0.01f;
+  return !(xb < b.cx_lo - margin || xb > b.cx_hi + margin || zb < b.cz_lo - margin || zb > b.cz_hi + margin);
+}
+
 // Pass 1, every voxel: zero TERMA and keep the voxels the beam may reach
 // (all voxels when intermediates are requested) on a compact list, so the
 // blocking/depth/TERMA pass runs on full warps.
@@ -502,27 +522,7 @@ __device__ __forceinline__ void cull_line(const GridDev& g, const BeamDev& b, fl
       pos[0] = px;
       pos[1] = py;
       pos[2] = voxel_centre(g.origin[2], g.spacing[2], z);
-      bool candidate = true;
-      if (b.cull_enable) {
-        const float np_ = b.vyf[0] * pos[0] + b.vyf[1] * pos[1] + b.vyf[2] * pos[2];
-        const float m0p = b.m0f[0] * pos[0] + b.m0f[1] * pos[1] + b.m0f[2] * pos[2];
-        const float m2p = b.m2f[0] * pos[0] + b.m2f[1] * pos[1] + b.m2f[2] * pos[2];
-        const float ndr = b.a_nS - np_;   // n . (S - p) = -depth
-        const float depth = -ndr;
-        if (depth > 0.2f * fabsf(b.a_K)) {
-          // one fast reciprocal: its ~2 ulp error is far inside the 0.01 cm
-          // margin, so the candidate set stays a superset of the beam
-          const float inv_depth = __fdividef(1.0f, depth);
-          const float si = -b.a_K * inv_depth;
-          const float xb = b.a_c0 + si * (b.a_m0S - m0p);
-          const float zb = b.a_c2 + si * (b.a_m2S - m2p);
-          const float lat = fmaxf(fabsf(b.a_m0S - m0p), fabsf(b.a_m2S - m2p)) * inv_depth;
-          const float margin = b.cull_margin_k * fabsf(b.a_K) * inv_depth * (1.0f + lat) + 0.01f;
-          if (xb < b.cx_lo - margin || xb > b.cx_hi + margin || zb < b.cz_lo - margin ||
-              zb > b.cz_hi + margin)
-            candidate = false;
-        }
-      }
+      const bool candidate = cull_candidate(b, pos);
       keep = candidate || all_voxels;
       if (zero_all) Tl[z] = 0.0f;
       if (!keep) {
@@ -572,10 +572,65 @@ __global__ void __launch_bounds__(256) cull_batch_kernel(const PrologueBeam* __r
             R.line_any, R.zero_all);
 }
 
-// Pass 2, listed voxels: blocked fraction, then (where the beam is not
-// fully blocked, or for every voxel when intermediates are requested)
-// radiological depth, oad, fluence, softening/horn and TERMA; TERMA support
-// box for the cone stage.
+// TERMA of voxel (x, y, z) centred at pos, v its index: blocked fraction, then
+// (where the beam is not fully blocked, or for every voxel when intermediates
+// are requested) radiological depth, oad, fluence, softening/horn and TERMA.
+// False when the voxel is blocked and nothing is written (Tv = 0).
+__device__ __forceinline__ bool terma_voxel(const float* __restrict__ rho, const GridDev& g, const BeamDev& b,
+                                            const SettingsDev& s, const Inter& inter, int all_voxels, int x, int y,
+                                            int z, int v, const float* pos, int& bad, float& Tv) {
+  Tv = 0.0f;
+  const double blocked = blocked_fraction(b, g, s.samples, pos, bad);
+  if (inter.blocked) inter.blocked[v] = blocked;
+  if (blocked == 0.0 && !all_voxels) {
+    if (inter.terma) inter.terma[v] = 0.0f;
+    return false;
+  }
+  float rd[3];
+  ray_to_source(b, pos, rd);
+  // ---- radiological depth (float32, exact mirror)
+  const float deff = radiological_depth(rho, g, x, y, z, rd);
+  // ---- off-axis distance (exact mirror)
+  float px = 0.0f, pz = 0.0f;
+  if (!project_exact(b, rd, px, pz)) bad = 1;
+  const float oad = __fsqrt_rn(fadd(fmul(px, px), fmul(pz, pz)));
+  // ---- fluence (float32 evaluation of the reference's float64 formula)
+  const float mag = __fsqrt_rn(fadd(fadd(fmul(rd[0], rd[0]), fmul(rd[1], rd[1])), fmul(rd[2], rd[2])));
+  const float sad = (float)b.sad;
+  const float ratio = sad / mag;
+  const float fpoint = s.sPri * (ratio * ratio);
+  const float r_ann = oad * s.zAnn / sad;
+  float fann = 0.0f;
+  if (r_ann >= s.rInner && r_ann <= s.rOuter) {
+    const float a = sad - s.zAnn, c = mag - s.zAnn;
+    fann = s.sAnn * (a * a) / (c * c);
+  }
+  const float oadc = oad < 2.0f ? 2.0f : oad;
+  const float r_exp = oadc * s.zExp / sad;
+  const float ae = sad - s.zExp, ce = mag - s.zExp;
+  const float fexp = s.sExp / r_exp * expf(-s.kExp * r_exp) * (ae * ae) / (ce * ce);
+  const float fluence = (float)((double)(fpoint + fann + fexp) * blocked);
+  // ---- softening and horn (reference host numpy, float32)
+  float fs = 1.0f;
+  if (oad < s.softLimit) fs = fdiv(1.0f, fsub(1.0f, fmul(s.softRatio, oad)));
+  const float fh = fadd(1.0f, fmul(oad, s.hornRatio));
+  // ---- TERMA (float32, reference order)
+  float terma = 0.0f;
+  for (int i = 0; i < s.n_energy; ++i) {
+    const float ex = expf(fmul(fmul(-s.mu[i], fs), deff));
+    terma = fadd(terma, fmul(fmul(fmul(fmul(fmul(s.w[i], fluence), ex), s.E[i]), s.mu[i]), fh));
+  }
+  Tv = d2f(dmul((double)terma, blocked));
+  if (inter.d_eff) inter.d_eff[v] = deff;
+  if (inter.oad) inter.oad[v] = oad;
+  if (inter.fluence) inter.fluence[v] = fluence;
+  if (inter.f_soften) inter.f_soften[v] = fs;
+  if (inter.f_horn) inter.f_horn[v] = fh;
+  if (inter.terma) inter.terma[v] = Tv;
+  return true;
+}
+
+// Pass 2, listed voxels: TERMA and its support box for the cone stage.
 // Entry e of a beam's list of count voxels; every lane of the warp calls it
 // (the box reduction is warp-wide).
 __device__ __forceinline__ void terma_entry(const float* __restrict__ rho, const GridDev& g, const BeamDev& b,
@@ -584,72 +639,19 @@ __device__ __forceinline__ void terma_entry(const float* __restrict__ rho, const
                                             int* __restrict__ aabb, int* __restrict__ flags) {
   {
     const bool live = e < count;
-    int x = 0, y = 0, z = 0, bad = 0, v = 0;
+    int x = 0, y = 0, z = 0, bad = 0;
     float Tv = 0.0f;
-    float pos[3] = {0.0f, 0.0f, 0.0f};
     if (live) {
-      v = list_v[e];
+      const int v = list_v[e];
       z = v % g.n[2];
       const int r = v / g.n[2];
       y = r % g.n[1];
       x = r / g.n[1];
-      pos[0] = voxel_centre(g.origin[0], g.spacing[0], x);
-      pos[1] = voxel_centre(g.origin[1], g.spacing[1], y);
-      pos[2] = voxel_centre(g.origin[2], g.spacing[2], z);
+      const float pos[3] = {voxel_centre(g.origin[0], g.spacing[0], x), voxel_centre(g.origin[1], g.spacing[1], y),
+                            voxel_centre(g.origin[2], g.spacing[2], z)};
+      if (terma_voxel(rho, g, b, s, inter, all_voxels, x, y, z, v, pos, bad, Tv))
+        T[((size_t)x * g.n[1] + y) * g.zp + z] = Tv;
     }
-    if (live) {
-      const double blocked = blocked_fraction(b, g, s.samples, pos, bad);
-      if (inter.blocked) inter.blocked[v] = blocked;
-      if (blocked == 0.0 && !all_voxels) {
-        if (inter.terma) inter.terma[v] = 0.0f;
-        goto next;
-      }
-      {
-      float rd[3];
-      ray_to_source(b, pos, rd);
-      // ---- radiological depth (float32, exact mirror)
-      const float deff = radiological_depth(rho, g, x, y, z, rd);
-      // ---- off-axis distance (exact mirror)
-      float px = 0.0f, pz = 0.0f;
-      if (!project_exact(b, rd, px, pz)) bad = 1;
-      const float oad = __fsqrt_rn(fadd(fmul(px, px), fmul(pz, pz)));
-      // ---- fluence (float32 evaluation of the reference's float64 formula)
-      const float mag = __fsqrt_rn(fadd(fadd(fmul(rd[0], rd[0]), fmul(rd[1], rd[1])), fmul(rd[2], rd[2])));
-      const float sad = (float)b.sad;
-      const float ratio = sad / mag;
-      const float fpoint = s.sPri * (ratio * ratio);
-      const float r_ann = oad * s.zAnn / sad;
-      float fann = 0.0f;
-      if (r_ann >= s.rInner && r_ann <= s.rOuter) {
-        const float a = sad - s.zAnn, c = mag - s.zAnn;
-        fann = s.sAnn * (a * a) / (c * c);
-      }
-      const float oadc = oad < 2.0f ? 2.0f : oad;
-      const float r_exp = oadc * s.zExp / sad;
-      const float ae = sad - s.zExp, ce = mag - s.zExp;
-      const float fexp = s.sExp / r_exp * expf(-s.kExp * r_exp) * (ae * ae) / (ce * ce);
-      const float fluence = (float)((double)(fpoint + fann + fexp) * blocked);
-      // ---- softening and horn (reference host numpy, float32)
-      float fs = 1.0f;
-      if (oad < s.softLimit) fs = fdiv(1.0f, fsub(1.0f, fmul(s.softRatio, oad)));
-      const float fh = fadd(1.0f, fmul(oad, s.hornRatio));
-      // ---- TERMA (float32, reference order)
-      float terma = 0.0f;
-      for (int i = 0; i < s.n_energy; ++i) {
-        const float ex = expf(fmul(fmul(-s.mu[i], fs), deff));
-        terma = fadd(terma, fmul(fmul(fmul(fmul(fmul(s.w[i], fluence), ex), s.E[i]), s.mu[i]), fh));
-      }
-      Tv = d2f(dmul((double)terma, blocked));
-      T[((size_t)x * g.n[1] + y) * g.zp + z] = Tv;
-      if (inter.d_eff) inter.d_eff[v] = deff;
-      if (inter.oad) inter.oad[v] = oad;
-      if (inter.fluence) inter.fluence[v] = fluence;
-      if (inter.f_soften) inter.f_soften[v] = fs;
-      if (inter.f_horn) inter.f_horn[v] = fh;
-      if (inter.terma) inter.terma[v] = Tv;
-      }
-    }
-  next:
     // ---- support box of T != 0 (the reference skips T == 0 sources), for the
     // gather's tap ranges.  Its six words share one L2 sector, and every chunk
     // of a beam in flight updated them: those adds took a sixth of the launch
@@ -745,6 +747,56 @@ __global__ void __launch_bounds__(256, 3) terma_batch_kernel(const PrologueBeam*
     terma_entry(R.rho, R.g, R.b, R.s, R.T, Inter{}, 0, count, ((c - base) << 5) + lane, R.list_v,
                 R.box ? R.aabb : nullptr, flags);
   }
+}
+
+// Cull and TERMA of a few small beams in one launch, a warp per (x, y) line:
+// the line test, the span of its candidate voxels, then TERMA of the span 32
+// voxels at a time and zeros beside it (on lines without candidates nothing:
+// line_any says so).  No list, no counters to reset, and the records come as a
+// kernel parameter: where the beams' voxels do not fill the SMs for long, the
+// time is that of launches and of one chunk's latency, and this needs one
+// launch and no copy instead of three and one.  flag_word gets the call's
+// epoch where a ray is parallel to the blocking plane.
+__global__ void __launch_bounds__(256, 3) prologue_fused_kernel(const __grid_constant__ FusedRecords A, int* flag_word,
+                                                                int epoch) {
+  const PrologueBeam& R = A.r[blockIdx.y];
+  const GridDev& g = R.g;
+  const BeamDev& b = R.b;
+  const int line = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (line >= g.n[0] * g.n[1]) return;   // whole warp
+  const int x = line / g.n[1], y = line - x * g.n[1], nz = g.n[2];
+  float pos[3] = {voxel_centre(g.origin[0], g.spacing[0], x), voxel_centre(g.origin[1], g.spacing[1], y), 0.0f};
+  int lo = nz, hi = -1;
+  if (!(b.cull_enable && line_outside(g, b, pos[0], pos[1])))
+    for (int z0 = 0; z0 < nz; z0 += 32) {
+      pos[2] = voxel_centre(g.origin[2], g.spacing[2], z0 + lane);
+      const unsigned m = __ballot_sync(0xffffffffu, z0 + lane < nz && cull_candidate(b, pos));
+      if (m) {
+        lo = min(lo, z0 + __ffs(m) - 1);
+        hi = z0 + 31 - __clz(m);
+      }
+    }
+  if (lane == 0) R.line_any[line] = hi >= 0;
+  if (hi < 0) return;
+  float* const T = R.T + (size_t)line * g.zp;
+  for (int z = lane; z < lo; z += 32) T[z] = 0.0f;
+  int bad = 0;
+  for (int z = lo + lane; z - lane <= hi; z += 32) {
+    float Tv = 0.0f;
+    pos[2] = voxel_centre(g.origin[2], g.spacing[2], z);
+    if (z <= hi && cull_candidate(b, pos))
+      terma_voxel(R.rho, g, b, R.s, Inter{}, 0, x, y, z, 0, pos, bad, Tv);
+    if (z < nz) T[z] = Tv;
+    __syncwarp();
+  }
+  const int end = lo + (hi - lo) / 32 * 32 + 32;
+  for (int z = end + lane; z < nz; z += 32) T[z] = 0.0f;
+  if (__any_sync(0xffffffffu, bad) && lane == 0) *flag_word = epoch;
+}
+
+void launch_prologue_fused(const FusedRecords& recs, int n_beams, long long max_lines, int* flag_word, int epoch,
+                           cudaStream_t st) {
+  prologue_fused_kernel<<<dim3((unsigned)((max_lines + 7) / 8), n_beams), 256, 0, st>>>(recs, flag_word, epoch);
 }
 
 // ----------------------------------------------------- beamlet adjoint --
