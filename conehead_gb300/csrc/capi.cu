@@ -681,6 +681,7 @@ BeamDev make_beam(const ch_beam& in, const ch_grid& g, int samples) {
     b.m0[k] = in.xform[k];
     b.m2[k] = in.xform[6 + k];
     b.srcf[k] = (float)in.src[k];
+    b.srcd[k] = b.srcf[k];
     b.vyf[k] = (float)in.vy[k];
     b.m0f[k] = (float)in.xform[k];
     b.m2f[k] = (float)in.xform[6 + k];
@@ -754,6 +755,8 @@ BeamDev make_beam(const ch_beam& in, const ch_grid& g, int samples) {
     P1 = std::max(P1, sum);
     D = std::max(D, std::sqrt(d2));
   }
+  // positions and lattice steps must fit one float64 significand exactly
+  if (P > std::ldexp(1.0, 22) * std::min(g.spacing[0], std::min(g.spacing[1], g.spacing[2]))) b.lat = 0;
   const double ray = std::sqrt(3.0) * P + D + 8.0 * P1;
   b.err_x = (float)(std::ldexp(1.0, -24) * (ray + 5.0 * std::max(std::fabs(m0S), std::fabs(m2S))));
   b.err_n = (float)(std::ldexp(1.0, -24) * (ray + 5.0 * std::fabs(nS)));

@@ -92,6 +92,7 @@ struct BeamDev {
   // exact mirror inputs
   double src[3], vy[3], m0[3], m2[3];   // m0/m2: transform rows 0 and 2
   double vyw;                           // v_y . float32(src), reference order
+  double srcd[3];                       // float32(src)
   float srcf[3], vyf[3], m0f[3], m2f[3], vywf;  // float32 copies (geom_f32 path)
   int geom_f32;
   // fast approximate projection: xb ~ c0 + si * (m0.S - m0.p), si = K / (n.S - n.p)
@@ -105,7 +106,7 @@ struct BeamDev {
   int brows, bcols, br0, bc0, full_rows, full_cols;
   int uniform;          // every crop value is 1.0
   // sub-sample lattice (blocked_fraction)
-  int lat;              // float64 source arrays: samples may be classified in float32
+  int lat;              // float64 source arrays on a sane grid: samples may be classified in float32
   int wraps;            // the crop holds the map's last row or column, which index -2000 reads
   float lat_n, lat_0, lat_2;   // largest |d nd|, |d x0|, |d x2| of a sub-sample from its voxel centre (cm)
   float err_x, err_n;   // float32 error bounds of x0 and nd against the reference's ray (cm)

@@ -66,7 +66,8 @@ __device__ __forceinline__ bool project_exact_mixed(const BeamDev& b, const floa
   const double si = ddiv(-b.vyw, ndotu);
   float pp[3];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) pp[k] = d2f(dadd(dadd((double)b.srcf[k], dmul(si, (double)rd[k])), 0.0));
+  // (the reference adds the plane point 0 as well: it could only turn -0 into 0)
+  for (int k = 0; k < 3; ++k) pp[k] = d2f(dadd(b.srcd[k], dmul(si, (double)rd[k])));
   px = d2f(dadd(dadd(dmul(b.m0[0], (double)pp[0]), dmul(b.m0[1], (double)pp[1])), dmul(b.m0[2], (double)pp[2])));
   pz = d2f(dadd(dadd(dmul(b.m2[0], (double)pp[0]), dmul(b.m2[1], (double)pp[1])), dmul(b.m2[2], (double)pp[2])));
   return true;
@@ -113,9 +114,12 @@ __device__ __forceinline__ bool sample_cell_exact(const BeamDev& b, const GridDe
   float ps[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    // ((pos - s/2) + off/2) + off*i, exact in float64, one rounding
-    const double v = dadd(dadd(dsub((double)pos[k], (double)g.spacing[k] * 0.5), (double)off[k] * 0.5),
-                          dmul((double)off[k], (double)ii[k]));
+    // ((pos - s/2) + off/2) + off*i, exact in float64 (a host check on the
+    // grid's extent stands behind lat), one rounding
+    const double v = b.lat ? __fma_rn((double)off[k], (double)((float)ii[k] + 0.5f),
+                                      dsub((double)pos[k], (double)(g.spacing[k] * 0.5f)))
+                           : dadd(dadd(dsub((double)pos[k], (double)g.spacing[k] * 0.5), (double)off[k] * 0.5),
+                                  dmul((double)off[k], (double)ii[k]));
     ps[k] = d2f(v);
   }
   float rd[3];
@@ -273,6 +277,79 @@ __device__ __forceinline__ void for_samples(const BeamDev& b, const float* off, 
   }
 }
 
+// Open samples (of 27) of a voxel that edges of a uniform crop cross, or -1 when
+// one lies within the error bound of an edge.  Against one edge, u < h + c0 for
+// instance, the test K x0 / nd < h is a sign of K x0 - h nd, which is linear
+// along the lattice: an add and a funnel shift per sample and edge that crosses
+// the voxel's bound (most voxels see one), and the smallest magnitude for the
+// error bound.  Its own rounding stays below 0.003 cells (six roundings of
+// terms up to 2200 |nd|).
+__device__ __forceinline__ int open_samples(const BeamDev& b, const float* off, const Centre& c) {
+  const float K = 100.0f * b.a_K;
+  const float tol = (c.delta + 0.003f) * (fabsf(c.nd) + b.lat_n);
+  unsigned open = 0x7ffffffu;
+  float least = 3.0e38f;
+#pragma unroll 1
+  for (int e = 0; e < 4; ++e) {
+    const bool along_u = e < 2;
+    const float sgn = (e & 1) ? -1.0f : 1.0f;
+    const float edge = along_u ? b.uc + sgn * b.uh : b.wc + sgn * b.wh;
+    if (fabsf((along_u ? c.u : c.w) - edge) > (along_u ? c.mu : c.mw)) continue;
+    const float h = edge - 100.0f * (along_u ? b.a_c0 : b.a_c2);
+    const float k = c.nd < 0.0f ? -sgn : sgn;         // F < 0 inside the edge
+    const float kK = k * K, kh = k * h;
+    float F = kK * (along_u ? c.x0 : c.x2) - kh * c.nd;
+    const float* m = along_u ? b.m0f : b.m2f;
+    const float fx = (kh * b.vyf[0] - kK * m[0]) * off[0], fy = (kh * b.vyf[1] - kK * m[1]) * off[1];
+    const float fz = (kh * b.vyf[2] - kK * m[2]) * off[2];
+    F -= fx + fy + fz;                                // sample (0, 0, 0)
+    unsigned in = 0;
+#pragma unroll
+    for (int ix = 0; ix < 3; ++ix)
+#pragma unroll
+      for (int iy = 0; iy < 3; ++iy) {
+        const float f0 = F + ((float)ix * fx + (float)iy * fy);
+#pragma unroll
+        for (int iz = 0; iz < 3; ++iz) {
+          const float f = f0 + (float)iz * fz;
+          in = __funnelshift_l(__float_as_uint(f), in, 1);   // its sign bit into bit 0
+          least = fminf(least, fabsf(f));
+        }
+      }
+    open &= in;
+  }
+  return least > tol ? __popc(open) : -1;
+}
+
+// Adds every sub-sample's transmission by add(v): value(u, w, amb) gives it from
+// the float32 coordinates or sets amb.  Ambiguous samples (up to 32 per voxel)
+// are taken after the loop, one per lane and round, so that the exact path runs
+// once or twice for a warp and not at every sample where one of its lanes needs
+// it; add's order does not matter.
+template <class V, class A>
+__device__ __forceinline__ void add_samples(const BeamDev& b, const GridDev& g, const float* pos, const float* off,
+                                            int S, const Centre& c, int& bad, V value, A add) {
+  const bool defer = S <= 3;
+  unsigned later = 0;
+  for_samples(b, off, S, c, [&](int ix, int iy, int iz, float u, float w) {
+    bool amb = false;
+    float v = value(u, w, amb);
+    if (amb) {
+      if (defer) {
+        later |= 1u << ((ix * S + iy) * S + iz);
+        return;
+      }
+      v = sample_exact(b, g, pos, off, ix, iy, iz, bad);
+    }
+    add(v);
+  });
+  while (later) {
+    const int i = __ffs(later) - 1;
+    later &= later - 1;
+    add(sample_exact(b, g, pos, off, i / (S * S), (i / S) % S, i % S, bad));
+  }
+}
+
 // floor of a coordinate clamped to +-1e6, as an integer: adding 1.5 2^23
 // rounding down leaves it in the low mantissa bits
 __device__ __forceinline__ int floor_int(float v) {
@@ -311,10 +388,17 @@ __device__ __forceinline__ double div_count(float v, double n, double inv_n) {
 // Both were bound by instruction issue: the field-edge voxels of a jaw field
 // were classified one per warp round, 27 lanes each (a chunk of 32 edge voxels
 // took 32 rounds), and a map's voxels went through those rounds and then again
-// through a per-lane loop with a float64 division per change of value.
-// Measured, whole call: nine MLC beams on 140 x 101 x 112 9425 -> 5060 us with
-// the fixed bound of 0.05 cells, 2660 us with delta and the walk below; one
-// 5 x 5 cm beam on 128^3 227 -> 194 us.
+// through a per-lane loop with a float64 division per change of value; then by
+// float64 issue (sums, exact samples).  Prologues, start of that work / now:
+// nine MLC beams on 140 x 101 x 112 8.59 / 1.22 ms, 64 mixed jaw beams 5.18 /
+// 2.69 ms, 32 beams 5 x 5 cm on 128^3 0.88 / 0.45 ms (the walk and the cull
+// below have their share; this function alone, last step: 1.69 -> 1.22, 2.94 ->
+// 2.69, 0.490 -> 0.446 ms).
+//
+// EXACT: the bits of the reference's float64 sum also for maps (where the
+// blocked fraction itself is returned); otherwise their samples are added in
+// 48 bits and divided once, ten times below a float32 rounding of the TERMA.
+template <bool EXACT>
 __device__ __forceinline__ double blocked_fraction(const BeamDev& b, const GridDev& g, int S, const float* pos,
                                                    int& bad) {
   Centre c;
@@ -327,38 +411,71 @@ __device__ __forceinline__ double blocked_fraction(const BeamDev& b, const GridD
   for (int k = 0; k < 3; ++k) off[k] = fdiv(g.spacing[k], (float)S);
   if (b.uniform) {
     if (du < -c.mu && dw < -c.mw) return c_unit_sum[S];
+    if (S == 3) {
+      const int n = open_samples(b, off, c);
+      if (n >= 0) return c_unit_partial[n];
+    }
     int n = 0;
-    for_samples(b, off, S, c, [&](int ix, int iy, int iz, float u, float w) {
-      const float d = fmaxf(fabsf(u - b.uc) - b.uh, fabsf(w - b.wc) - b.wh);
-      if (fabsf(d) > c.delta)
-        n += d < 0.0f ? 1 : 0;
-      else
-        n += sample_exact(b, g, pos, off, ix, iy, iz, bad) == 1.0f ? 1 : 0;
-    });
+    add_samples(b, g, pos, off, S, c, bad,
+                [&](float u, float w, bool& amb) {
+                  const float d = fmaxf(fabsf(u - b.uc) - b.uh, fabsf(w - b.wc) - b.wh);
+                  amb = fabsf(d) <= c.delta;
+                  return d < 0.0f ? 1.0f : 0.0f;
+                },
+                [&](float v) { n += v == 1.0f ? 1 : 0; });
     if (S == 3) return c_unit_partial[n];
     const double q = c_inv_count[S];
     double acc = 0.0;
     for (int i = 0; i < n; ++i) acc = dadd(acc, q);
     return acc;
   }
+  // Coordinates are within the crop and the bound around it: floor by the
+  // magic addition needs no clamp.
+  const float clear = 0.5f - c.delta;
+  auto value = [&](float u, float w, bool& amb) {
+    const float mu = __fadd_rd(u, 12582912.0f), mw = __fadd_rd(w, 12582912.0f);
+    const int i = __float_as_int(mu) - 0x4b400000, k = __float_as_int(mw) - 0x4b400000;
+    const float v = map_value(b, i, k);
+    const float du = (u - (mu - 12582912.0f)) - 0.5f, dw = (w - (mw - 12582912.0f)) - 0.5f;
+    if (fmaxf(fabsf(du), fabsf(dw)) >= clear) {
+      const int i1 = fabsf(du) >= clear ? i + (du < 0.0f ? -1 : 1) : i;
+      const int k1 = fabsf(dw) >= clear ? k + (dw < 0.0f ? -1 : 1) : k;
+      const float v1 = map_value(b, i1, k), v2 = map_value(b, i, k1), v3 = map_value(b, i1, k1);
+      amb = v1 != v || v2 != v || v3 != v;
+    }
+    return v;
+  };
   const double count = (double)(S * S * S), inv = c_inv_count[S];
-  double acc = 0.0, q = 0.0;
-  float last = 0.0f;
-  for_samples(b, off, S, c, [&](int ix, int iy, int iz, float u, float w) {
-    const int i0 = floor_int(u - c.delta), i1 = floor_int(u + c.delta);
-    const int k0 = floor_int(w - c.delta), k1 = floor_int(w + c.delta);
-    float v = map_value(b, i0, k0);
-    if (i0 != i1 || k0 != k1) {
-      const float v1 = map_value(b, i1, k0), v2 = map_value(b, i0, k1), v3 = map_value(b, i1, k1);
-      if (v1 != v || v2 != v || v3 != v) v = sample_exact(b, g, pos, off, ix, iy, iz, bad);
+  if (EXACT) {
+    // the reference's float64 sum, share by share (one value and its quotient kept)
+    double acc = 0.0, q = 0.0;
+    float last = 0.0f;
+    for_samples(b, off, S, c, [&](int ix, int iy, int iz, float u, float w) {
+      bool amb = false;
+      float v = value(u, w, amb);
+      if (amb) v = sample_exact(b, g, pos, off, ix, iy, iz, bad);
+      if (v != last) {
+        last = v;
+        q = div_count(v, count, inv);
+      }
+      if (v != 0.0f) acc = dadd(acc, q);
+    });
+    return acc;
+  }
+  // ones are counted, other values summed in float32 pairs (48 bits, Knuth's
+  // two-sum): float64 adds issue at two lanes per clock and SM
+  int ones = 0;
+  float hi = 0.0f, lo = 0.0f;
+  add_samples(b, g, pos, off, S, c, bad, value, [&](float v) {
+    ones += v == 1.0f ? 1 : 0;
+    if (v != 0.0f && v != 1.0f) {
+      const float t = fadd(hi, v), bb = fsub(t, hi);
+      lo = fadd(lo, fadd(fsub(hi, fsub(t, bb)), fsub(v, bb)));
+      hi = t;
     }
-    if (v != last) {
-      last = v;
-      q = div_count(v, count, inv);
-    }
-    if (v != 0.0f) acc = dadd(acc, q);
   });
-  return acc;
+  if (hi == 0.0f && lo == 0.0f && S == 3) return c_unit_partial[ones];
+  return ddiv(dadd(dadd((double)hi, (double)lo), (double)ones), count);
 }
 
 // ------------------------------------------------------------------ DDA --
@@ -645,11 +762,12 @@ __global__ void __launch_bounds__(256) cull_batch_kernel(const PrologueBeam* __r
 // (where the beam is not fully blocked, or for every voxel when intermediates
 // are requested) radiological depth, oad, fluence, softening/horn and TERMA.
 // False when the voxel is blocked and nothing is written (Tv = 0).
+template <bool EXACT>
 __device__ __forceinline__ bool terma_voxel(const float* __restrict__ rho, const GridDev& g, const BeamDev& b,
                                             const SettingsDev& s, const Inter& inter, int all_voxels, int x, int y,
                                             int z, int v, const float* pos, int& bad, float& Tv) {
   Tv = 0.0f;
-  const double blocked = blocked_fraction(b, g, s.samples, pos, bad);
+  const double blocked = blocked_fraction<EXACT>(b, g, s.samples, pos, bad);
   if (inter.blocked) inter.blocked[v] = blocked;
   if (blocked == 0.0 && !all_voxels) {
     if (inter.terma) inter.terma[v] = 0.0f;
@@ -678,7 +796,11 @@ __device__ __forceinline__ bool terma_voxel(const float* __restrict__ rho, const
   const float r_exp = oadc * s.zExp / sad;
   const float ae = sad - s.zExp, ce = mag - s.zExp;
   const float fexp = s.sExp / r_exp * expf(-s.kExp * r_exp) * (ae * ae) / (ce * ce);
-  const float fluence = (float)((double)(fpoint + fann + fexp) * blocked);
+  // a product with the sum of S^3 equal shares (1 within a few 2^-53) rounds
+  // to the float32 factor itself
+  const bool open = blocked == c_unit_sum[s.samples];
+  float fluence = fpoint + fann + fexp;
+  if (!open) fluence = (float)((double)fluence * blocked);
   // ---- softening and horn (reference host numpy, float32)
   float fs = 1.0f;
   if (oad < s.softLimit) fs = fdiv(1.0f, fsub(1.0f, fmul(s.softRatio, oad)));
@@ -689,7 +811,7 @@ __device__ __forceinline__ bool terma_voxel(const float* __restrict__ rho, const
     const float ex = expf(fmul(fmul(-s.mu[i], fs), deff));
     terma = fadd(terma, fmul(fmul(fmul(fmul(fmul(s.w[i], fluence), ex), s.E[i]), s.mu[i]), fh));
   }
-  Tv = d2f(dmul((double)terma, blocked));
+  Tv = open ? terma : d2f(dmul((double)terma, blocked));
   if (inter.d_eff) inter.d_eff[v] = deff;
   if (inter.oad) inter.oad[v] = oad;
   if (inter.fluence) inter.fluence[v] = fluence;
@@ -702,6 +824,7 @@ __device__ __forceinline__ bool terma_voxel(const float* __restrict__ rho, const
 // Pass 2, listed voxels: TERMA and its support box for the cone stage.
 // Entry e of a beam's list of count voxels; every lane of the warp calls it
 // (the box reduction is warp-wide).
+template <bool EXACT>
 __device__ __forceinline__ void terma_entry(const float* __restrict__ rho, const GridDev& g, const BeamDev& b,
                                             const SettingsDev& s, float* __restrict__ T, const Inter& inter,
                                             int all_voxels, int count, int e, const int* __restrict__ list_v,
@@ -718,7 +841,7 @@ __device__ __forceinline__ void terma_entry(const float* __restrict__ rho, const
       x = r / g.n[1];
       const float pos[3] = {voxel_centre(g.origin[0], g.spacing[0], x), voxel_centre(g.origin[1], g.spacing[1], y),
                             voxel_centre(g.origin[2], g.spacing[2], z)};
-      if (terma_voxel(rho, g, b, s, inter, all_voxels, x, y, z, v, pos, bad, Tv))
+      if (terma_voxel<EXACT>(rho, g, b, s, inter, all_voxels, x, y, z, v, pos, bad, Tv))
         T[((size_t)x * g.n[1] + y) * g.zp + z] = Tv;
     }
     // ---- support box of T != 0 (the reference skips T == 0 sources), for the
@@ -761,7 +884,7 @@ __device__ __forceinline__ void terma_body(const float* __restrict__ rho, const 
   const int count = *list_count;
   const int rounds = (count + blockDim.x * n_ctas - 1) / (blockDim.x * n_ctas);
   for (int it = 0; it < rounds; ++it)
-    terma_entry(rho, g, b, s, T, inter, all_voxels, count, (it * n_ctas + cta) * blockDim.x + threadIdx.x,
+    terma_entry<true>(rho, g, b, s, T, inter, all_voxels, count, (it * n_ctas + cta) * blockDim.x + threadIdx.x,
                 list_v, aabb, flags);
 }
 
@@ -813,7 +936,7 @@ __global__ void __launch_bounds__(256, 3) terma_batch_kernel(const PrologueBeam*
       __syncwarp();
       cur = beam;
     }
-    terma_entry(R.rho, R.g, R.b, R.s, R.T, Inter{}, 0, count, ((c - base) << 5) + lane, R.list_v,
+    terma_entry<false>(R.rho, R.g, R.b, R.s, R.T, Inter{}, 0, count, ((c - base) << 5) + lane, R.list_v,
                 R.box ? R.aabb : nullptr, flags);
   }
 }
@@ -854,7 +977,7 @@ __global__ void __launch_bounds__(256, 3) prologue_fused_kernel(const __grid_con
     float Tv = 0.0f;
     pos[2] = voxel_centre(g.origin[2], g.spacing[2], z);
     if (z <= hi && cull_candidate(b, pos))
-      terma_voxel(R.rho, g, b, R.s, Inter{}, 0, x, y, z, 0, pos, bad, Tv);
+      terma_voxel<false>(R.rho, g, b, R.s, Inter{}, 0, x, y, z, 0, pos, bad, Tv);
     if (z < nz) T[z] = Tv;
     __syncwarp();
   }
@@ -982,7 +1105,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) blocked_adjoint_kernel(GridDev g,
     int id0 = 0;           // beamlet (a, c), which may lie outside the grid
     double gv = 0.0;
     if (t != 0.0f && tb != 0.0f) {
-      const double blocked = blocked_fraction(b, g, S, pos, bad);
+      const double blocked = blocked_fraction<false>(b, g, S, pos, bad);
       Centre c;
       if (blocked > 0.0) {
         gv = (double)tb * 2.0 * (double)t / blocked * inv;
