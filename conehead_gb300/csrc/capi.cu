@@ -1887,6 +1887,7 @@ ch_status ch_dose_adjoint(ch_plan* P, const ch_grid* grid, const float* rho, int
   CH_CUDA(P->aabb.ensure(16 * sizeof(int)));
   CH_CUDA(P->counters.ensure(need.bytes[2]));
   CH_CUDA(P->list_v.ensure(need.bytes[7]));
+  CH_CUDA(P->pro_beams.ensure(sizeof(PrologueBeam)));
   CH_CUDA(P->adj_out.ensure(N * sizeof(float)));
   CH_CUDA(P->adj_w.ensure((size_t)bl->rows * bl->cols * sizeof(double)));
   int* box = P->aabb.as<int>();          // [0..7] TERMA box + list count, [8..15] input box
@@ -1896,9 +1897,22 @@ ch_status ch_dose_adjoint(ch_plan* P, const ch_grid* grid, const float* rho, int
   const SettingsDev sd = make_settings(*settings);
   P->flags_by_epoch = false;
   launch_init_scratch(box, 2, counters, s);
-  // forward prologue: TERMA, its box and the list of voxels the beam reaches
-  launch_prologue(rho, g, b, sd, P->T.as<float>(), Inter{}, 0, box, !spec_batch(P, 1, grid), P->list_v.as<int>(),
-                  P->n_sm, flags, s, P->tuning.terma_ctas_per_sm);
+  // forward prologue: TERMA, its box (gather) and the list of voxels the beam reaches
+  const bool gather = !spec_batch(P, 1, grid);
+  PrologueBeam rec;
+  std::memset(&rec, 0, sizeof(rec));
+  rec.g = g;
+  rec.b = b;
+  rec.s = sd;
+  rec.rho = rho;
+  rec.T = P->T.as<float>();
+  rec.aabb = box;
+  rec.list_v = P->list_v.as<int>();
+  rec.line_any = reinterpret_cast<unsigned char*>(P->list_v.as<int>() + (N + 63) / 64 * 64);
+  rec.zero_all = rec.box = gather ? 1 : 0;
+  if ((st = stage_records(P, {Seg{P->pro_beams.p, &rec, sizeof(rec)}}, s)) != CH_OK) return st;
+  launch_prologue_batch(P->pro_beams.as<PrologueBeam>(), 1, (long long)N, (long long)g.n[0] * g.n[1], P->n_sm, flags,
+                        counters + 4, s, P->tuning.terma_ctas_per_sm);
   CH_CUDA(cudaGetLastError());
   // transposed cone: dL/dT = C^T dL/dD, only where TERMA is nonzero
   float* tbar = grad_terma ? grad_terma : P->adj_out.as<float>();

@@ -277,48 +277,80 @@ __device__ __forceinline__ void for_samples(const BeamDev& b, const float* off, 
   }
 }
 
-// Open samples (of 27) of a voxel that edges of a uniform crop cross, or -1 when
-// one lies within the error bound of an edge.  Against one edge, u < h + c0 for
-// instance, the test K x0 / nd < h is a sign of K x0 - h nd, which is linear
-// along the lattice: an add and a funnel shift per sample and edge that crosses
-// the voxel's bound (most voxels see one), and the smallest magnitude for the
-// error bound.  Its own rounding stays below 0.003 cells (six roundings of
-// terms up to 2200 |nd|).
-__device__ __forceinline__ int open_samples(const BeamDev& b, const float* off, const Centre& c) {
+// The 27 samples of a voxel (bit 26 - (9 ix + 3 iy + iz)) on one side of a line of
+// the block map, u = edge or w = edge: sgn * (coordinate - edge) < 0.  The test
+// K x0 / nd < h is a sign of K x0 - h nd, which is linear along the lattice: an
+// add and a funnel shift per sample.  near gets the samples within the error
+// bound of the line, which the caller decides exactly; the form's own rounding
+// stays below 0.003 cells (six roundings of terms up to 2200 |nd|).
+constexpr unsigned ALL_27 = 0x7ffffffu;
+__device__ __forceinline__ unsigned below_edge(const BeamDev& b, const float* off, const Centre& c, bool along_u,
+                                               float edge, float sgn, unsigned& near) {
   const float K = 100.0f * b.a_K;
-  const float tol = (c.delta + 0.003f) * (fabsf(c.nd) + b.lat_n);
-  unsigned open = 0x7ffffffu;
+  const float h = edge - 100.0f * (along_u ? b.a_c0 : b.a_c2);
+  const float k = c.nd < 0.0f ? -sgn : sgn;
+  const float kK = k * K, kh = k * h;
+  float F = kK * (along_u ? c.x0 : c.x2) - kh * c.nd;
+  const float* m = along_u ? b.m0f : b.m2f;
+  const float fx = (kh * b.vyf[0] - kK * m[0]) * off[0], fy = (kh * b.vyf[1] - kK * m[1]) * off[1];
+  const float fz = (kh * b.vyf[2] - kK * m[2]) * off[2];
+  F -= fx + fy + fz;                                // sample (0, 0, 0)
+  unsigned in = 0;
   float least = 3.0e38f;
+#pragma unroll
+  for (int ix = 0; ix < 3; ++ix)
+#pragma unroll
+    for (int iy = 0; iy < 3; ++iy) {
+      const float f0 = F + ((float)ix * fx + (float)iy * fy);
+#pragma unroll
+      for (int iz = 0; iz < 3; ++iz) {
+        const float f = f0 + (float)iz * fz;
+        in = __funnelshift_l(__float_as_uint(f), in, 1);   // its sign bit into bit 0
+        least = fminf(least, fabsf(f));
+      }
+    }
+  const float tol = (c.delta + 0.003f) * (fabsf(c.nd) + b.lat_n);
+  if (!(least > tol)) {
+    unsigned n = 0;
+#pragma unroll 1
+    for (int ix = 0; ix < 3; ++ix)
+#pragma unroll
+      for (int q = 0; q < 9; ++q) {
+        const float f = F + ((float)ix * fx + (float)(q / 3) * fy) + (float)(q % 3) * fz;
+        n = (n << 1) | (fabsf(f) > tol ? 0u : 1u);
+      }
+    near |= n;
+  }
+  return in;
+}
+
+// Calls f(bit, ix, iy, iz) for every sample of a mask of below_edge's.
+template <class F>
+__device__ __forceinline__ void for_mask(unsigned mask, F f) {
+  while (mask) {
+    const int bit = __ffs(mask) - 1, i = 26 - bit;
+    mask &= mask - 1;
+    f(1u << bit, i / 9, (i / 3) % 3, i % 3);
+  }
+}
+
+// Open samples (of 27) of a voxel that edges of a uniform crop cross (most
+// voxels see one).
+__device__ __forceinline__ int open_samples(const BeamDev& b, const GridDev& g, const float* pos, const float* off,
+                                            const Centre& c, int& bad) {
+  unsigned open = ALL_27, near = 0;
 #pragma unroll 1
   for (int e = 0; e < 4; ++e) {
     const bool along_u = e < 2;
     const float sgn = (e & 1) ? -1.0f : 1.0f;
     const float edge = along_u ? b.uc + sgn * b.uh : b.wc + sgn * b.wh;
-    if (fabsf((along_u ? c.u : c.w) - edge) > (along_u ? c.mu : c.mw)) continue;
-    const float h = edge - 100.0f * (along_u ? b.a_c0 : b.a_c2);
-    const float k = c.nd < 0.0f ? -sgn : sgn;         // F < 0 inside the edge
-    const float kK = k * K, kh = k * h;
-    float F = kK * (along_u ? c.x0 : c.x2) - kh * c.nd;
-    const float* m = along_u ? b.m0f : b.m2f;
-    const float fx = (kh * b.vyf[0] - kK * m[0]) * off[0], fy = (kh * b.vyf[1] - kK * m[1]) * off[1];
-    const float fz = (kh * b.vyf[2] - kK * m[2]) * off[2];
-    F -= fx + fy + fz;                                // sample (0, 0, 0)
-    unsigned in = 0;
-#pragma unroll
-    for (int ix = 0; ix < 3; ++ix)
-#pragma unroll
-      for (int iy = 0; iy < 3; ++iy) {
-        const float f0 = F + ((float)ix * fx + (float)iy * fy);
-#pragma unroll
-        for (int iz = 0; iz < 3; ++iz) {
-          const float f = f0 + (float)iz * fz;
-          in = __funnelshift_l(__float_as_uint(f), in, 1);   // its sign bit into bit 0
-          least = fminf(least, fabsf(f));
-        }
-      }
-    open &= in;
+    if (fabsf((along_u ? c.u : c.w) - edge) <= (along_u ? c.mu : c.mw))
+      open &= below_edge(b, off, c, along_u, edge, sgn, near);
   }
-  return least > tol ? __popc(open) : -1;
+  for_mask(near, [&](unsigned bit, int ix, int iy, int iz) {
+    open = sample_exact(b, g, pos, off, ix, iy, iz, bad) == 1.0f ? open | bit : open & ~bit;
+  });
+  return __popc(open);
 }
 
 // Adds every sub-sample's transmission by add(v): value(u, w, amb) gives it from
@@ -411,10 +443,7 @@ __device__ __forceinline__ double blocked_fraction(const BeamDev& b, const GridD
   for (int k = 0; k < 3; ++k) off[k] = fdiv(g.spacing[k], (float)S);
   if (b.uniform) {
     if (du < -c.mu && dw < -c.mw) return c_unit_sum[S];
-    if (S == 3) {
-      const int n = open_samples(b, off, c);
-      if (n >= 0) return c_unit_partial[n];
-    }
+    if (S == 3) return c_unit_partial[open_samples(b, g, pos, off, c, bad)];
     int n = 0;
     add_samples(b, g, pos, off, S, c, bad,
                 [&](float u, float w, bool& amb) {
@@ -423,7 +452,6 @@ __device__ __forceinline__ double blocked_fraction(const BeamDev& b, const GridD
                   return d < 0.0f ? 1.0f : 0.0f;
                 },
                 [&](float v) { n += v == 1.0f ? 1 : 0; });
-    if (S == 3) return c_unit_partial[n];
     const double q = c_inv_count[S];
     double acc = 0.0;
     for (int i = 0; i < n; ++i) acc = dadd(acc, q);
@@ -1049,35 +1077,39 @@ __device__ __forceinline__ int beamlet_index(float v, float cell, float inv_cell
 // dL/dw for blocked(v) = sum_s w[beamlet(s)] / S^3 and T = blocked^2 * H
 // (fluence and TERMA each carry one factor of blocked): over the voxels of
 // the prologue's list with T != 0, g(v) = tbar(v) * 2 T(v) / blocked(v) is
-// spread over the beamlets of its S^3 sub-samples.  Per-CTA float64
-// histograms in shared memory, one global float64 add per touched beamlet.
+// spread over the beamlets of its S^3 sub-samples, in float64.
 //
-// One voxel per lane, 32 consecutive entries of the list per warp.  A voxel
-// whose samples span at most 2 x 2 beamlets (beamlets wider than its shadow
-// on the block plane) counts its samples per beamlet in four byte fields, and
-// the warp adds each beamlet's total once: float64 adds in shared memory are
-// compare-and-swap loops, and a warp's voxels lie in the same few beamlets, so
-// one add per sample serialised 32 ways.  Smaller beamlets add per change of
-// beamlet.
-constexpr int ADJ_THREADS = 512;
-__global__ void __launch_bounds__(ADJ_THREADS) blocked_adjoint_kernel(GridDev g, BeamDev b, BeamletDev bl, int S,
-                                                                      const float* __restrict__ T,
-                                                                      const float* __restrict__ tbar,
-                                                                      const int* __restrict__ list_count,
-                                                                      const int* __restrict__ list_v,
-                                                                      double* __restrict__ wbar,
-                                                                      int* __restrict__ flags) {
-  extern __shared__ double hist[];
+// One voxel per lane, 32 consecutive entries of the list per warp.  With 3
+// samples per axis and a shadow on at most 2 x 2 beamlets (a, c) .. (a + 1,
+// c + 1), the samples in each are popcounts of two side tests (below_edge), and
+// blocked is the counts' mean of the crop's values there.  Runs of lanes with
+// the same beamlet (neighbours along z) are summed first, as float32 pairs, and
+// add once, to L2: a histogram in shared memory adds float64 by compare-and-swap
+// loops that the SM's warps, all at the same few beamlets, make each other
+// repeat, and its flush costs as many global adds as this.  Other voxels go
+// sample by sample and add per change of beamlet.
+//
+// 40 x 40 beamlets of 0.5 cm on 128^3 (one million voxels): one warp-wide sum
+// per distinct beamlet 988 us (a line of 32 voxels crosses 16 of them; 128
+// registers, one CTA per SM), runs into a shared histogram 420 us, into L2 390 us,
+// with ambiguous samples decided one by one instead of the whole voxel 167 us.
+constexpr int ADJ_THREADS = 256;
+__global__ void __launch_bounds__(ADJ_THREADS, 3) blocked_adjoint_kernel(const __grid_constant__ GridDev g,
+                                                                         const __grid_constant__ BeamDev b,
+                                                                         const BeamletDev bl, int S,
+                                                                         const float* __restrict__ T,
+                                                                         const float* __restrict__ tbar,
+                                                                         const int* __restrict__ list_count,
+                                                                         const int* __restrict__ list_v,
+                                                                         double* __restrict__ wbar,
+                                                                         int* __restrict__ flags) {
   const unsigned full = 0xffffffffu;
-  const int nb = bl.rows * bl.cols, lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) hist[i] = 0.0;
-  __syncthreads();
+  const int lane = threadIdx.x & 31;
   const int count = *list_count;
   int bad = 0;
   float off[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) off[k] = fdiv(g.spacing[k], (float)S);
-  const double inv = 1.0 / ((double)S * (double)S * (double)S);
   const float cr = (float)bl.cell_rows, cc = (float)bl.cell_cols;
   const float icr = 1.0f / cr, icc = 1.0f / cc;
   // cell coordinate of the beamlet grid's first row and column
@@ -1103,49 +1135,69 @@ __global__ void __launch_bounds__(ADJ_THREADS) blocked_adjoint_kernel(GridDev g,
     }
     unsigned cnt = 0;      // samples in beamlets (a, c), (a, c + 1), (a + 1, c), (a + 1, c + 1), a byte each
     int id0 = 0;           // beamlet (a, c), which may lie outside the grid
-    double gv = 0.0;
+    float ghi = 0.0f, glo = 0.0f;   // g(v) / S^3
     if (t != 0.0f && tb != 0.0f) {
-      const double blocked = blocked_fraction<false>(b, g, S, pos, bad);
       Centre c;
-      if (blocked > 0.0) {
-        gv = (double)tb * 2.0 * (double)t / blocked * inv;
-        const bool lat = whole && lattice_centre(b, pos, c);
-        int a = 0, k = 0;
-        bool four = false;
-        if (lat) {
-          a = floor_int((c.u - c.mu - u0) * icr - 1e-3f);
-          k = floor_int((c.w - c.mw - w0) * icc - 1e-3f);
-          four = S <= 6 && floor_int((c.u + c.mu - u0) * icr + 1e-3f) <= a + 1 &&
-                 floor_int((c.w + c.mw - w0) * icc + 1e-3f) <= k + 1;
+      const bool lat = whole && lattice_centre(b, pos, c);
+      bool done = false;
+      if (lat && S == 3) {
+        const int a = floor_int((c.u - c.mu - u0) * icr - 1e-3f), k = floor_int((c.w - c.mw - w0) * icc - 1e-3f);
+        const float eu = u0 + (float)(a + 1) * cr, ew = w0 + (float)(k + 1) * cc;   // the lines between them
+        if (c.u + c.mu < eu + cr && c.w + c.mw < ew + cc) {
+          unsigned near = 0;
+          unsigned in_u = c.u + c.mu < eu ? ALL_27 : below_edge(b, off, c, true, eu, 1.0f, near);
+          unsigned in_w = c.w + c.mw < ew ? ALL_27 : below_edge(b, off, c, false, ew, 1.0f, near);
+          for_mask(near, [&](unsigned bit, int ix, int iy, int iz) {
+            int fi, fk;
+            if (!sample_cell_exact(b, g, pos, off, ix, iy, iz, bad, fi, fk)) return;
+            in_u = (float)fi < eu ? in_u | bit : in_u & ~bit;
+            in_w = (float)fk < ew ? in_w | bit : in_w & ~bit;
+          });
+          done = true;
           id0 = a * bl.cols + k;
+          double sum = 0.0;
+#pragma unroll
+          for (int f = 0; f < 4; ++f) {
+            const int i = a + (f >> 1), j = k + (f & 1);
+            if (i < 0 || i >= bl.rows || j < 0 || j >= bl.cols) continue;
+            const int n = __popc(((f & 2) ? ~in_u & ALL_27 : in_u) & ((f & 1) ? ~in_w & ALL_27 : in_w));
+            cnt |= (unsigned)n << (8 * f);
+            if (n)
+              sum = __fma_rn((double)n, (double)__ldg(b.block + (size_t)(i * bl.cell_rows) * b.bcols + j * bl.cell_cols),
+                             sum);
+          }
+          // 2 t tb / S^3 / blocked with blocked = sum / S^3
+          const double gv = sum > 0.0 ? 2.0 * (double)t * (double)tb / sum : 0.0;
+          ghi = d2f(gv);
+          glo = d2f(gv - (double)ghi);
         }
-        if (lat) {
-          int cur = -1, n = 0;
+      }
+      if (!done) {
+        const double blocked = blocked_fraction<false>(b, g, S, pos, bad);
+        const double gv = blocked > 0.0 ? (double)tb * 2.0 * (double)t / blocked / ((double)S * S * S) : 0.0;
+        int cur = -1, n = 0;
+        auto sample = [&](int id) {
+          if (id == cur) {
+            ++n;
+          } else if (id >= 0) {
+            if (n) atomicAdd(wbar + cur, gv * (double)n);
+            cur = id;
+            n = 1;
+          }
+        };
+        if (gv == 0.0) {
+        } else if (lat) {
           for_samples(b, off, S, c, [&](int ix, int iy, int iz, float u, float w) {
             bool amb = false;
-            int i = beamlet_index(u - u0, cr, icr, bl.rows, c.delta, amb);
-            int j = beamlet_index(w - w0, cc, icc, bl.cols, c.delta, amb);
+            const int i = beamlet_index(u - u0, cr, icr, bl.rows, c.delta, amb);
+            const int j = beamlet_index(w - w0, cc, icc, bl.cols, c.delta, amb);
+            int id = (i < 0 || j < 0) ? -1 : i * bl.cols + j;
             if (amb) {
               int fi, fk;
-              int id = -1;
-              if (sample_cell_exact(b, g, pos, off, ix, iy, iz, bad, fi, fk)) id = beamlet_of(b, bl, fi, fk);
-              i = id < 0 ? -1 : id / bl.cols;
-              j = id < 0 ? -1 : id - i * bl.cols;
+              id = sample_cell_exact(b, g, pos, off, ix, iy, iz, bad, fi, fk) ? beamlet_of(b, bl, fi, fk) : -1;
             }
-            if (i < 0 || j < 0) return;
-            if (four && (unsigned)(i - a) < 2u && (unsigned)(j - k) < 2u) {
-              cnt += 1u << (8 * (2 * (i - a) + (j - k)));
-            } else {
-              const int id = i * bl.cols + j;
-              if (id != cur) {
-                if (n) atomicAdd(hist + cur, gv * (double)n);
-                cur = id;
-                n = 0;
-              }
-              ++n;
-            }
+            sample(id);
           });
-          if (n) atomicAdd(hist + cur, gv * (double)n);
         } else {
           for (int ix = 0; ix < S; ++ix)
             for (int iy = 0; iy < S; ++iy)
@@ -1153,47 +1205,42 @@ __global__ void __launch_bounds__(ADJ_THREADS) blocked_adjoint_kernel(GridDev g,
                 const float rx = off[0] * ((float)ix + 0.5f) - g.spacing[0] * 0.5f;
                 const float ry = off[1] * ((float)iy + 0.5f) - g.spacing[1] * 0.5f;
                 const float rz = off[2] * ((float)iz + 0.5f) - g.spacing[2] * 0.5f;
-                const int id = sample_beamlet(b, bl, g, pos, off, rx, ry, rz, ix, iy, iz, bad);
-                if (id >= 0) atomicAdd(hist + id, gv);
+                sample(sample_beamlet(b, bl, g, pos, off, rx, ry, rz, ix, iy, iz, bad));
               }
         }
+        if (n) atomicAdd(wbar + cur, gv * (double)n);
       }
     }
-    // the warp's totals, one add per beamlet and field (only beamlets of the grid hold counts)
+    // byte fields: suffix sums over runs of lanes with the same beamlet, added by each run's first lane
+    const int next_id = __shfl_down_sync(full, id0, 1);
+    const unsigned same_next = __ballot_sync(full, lane < 31 && id0 == next_id);   // lane and lane + 1
+    const int run = __clz(__brev(~(same_next >> lane)));           // lanes of the run after this one
+    const bool first = lane == 0 || !((same_next >> (lane - 1)) & 1u);
 #pragma unroll 1
     for (int f = 0; f < 4; ++f) {
-      const int n = (int)((cnt >> (8 * f)) & 255u);
-      const int id = id0 + (f >> 1) * bl.cols + (f & 1);
-      unsigned todo = __ballot_sync(full, n > 0);
-      while (todo) {
-        const int lead = __ffs(todo) - 1;
-        const int lid = __shfl_sync(full, id, lead);
-        const bool mine = n > 0 && id == lid;
-        double sum = mine ? gv * (double)n : 0.0;
+      const float n = (float)((cnt >> (8 * f)) & 255u);
+      if (!__any_sync(full, n > 0.0f)) continue;
+      float hi = ghi * n, lo = __fmaf_rn(ghi, n, -hi) + glo * n;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(full, sum, o);
-        if (lane == lead) atomicAdd(hist + lid, sum);
-        todo &= ~__ballot_sync(full, mine);
+      for (int o = 1; o < 32; o <<= 1) {
+        const float h2 = __shfl_down_sync(full, hi, o), l2 = __shfl_down_sync(full, lo, o);
+        if (o <= run) {
+          const float t2 = fadd(hi, h2), bb = fsub(t2, hi);
+          lo = fadd(fadd(lo, l2), fadd(fsub(hi, fsub(t2, bb)), fsub(h2, bb)));
+          hi = t2;
+        }
       }
+      const double sum = fabsf(hi) <= 3.4028234e38f ? (double)hi + (double)lo : (double)hi;
+      if (first && sum != 0.0) atomicAdd(wbar + id0 + (f >> 1) * bl.cols + (f & 1), sum);
     }
   }
   if (__any_sync(full, bad) && lane == 0) atomicOr(flags, FLAG_PARALLEL_RAY);
-  __syncthreads();
-  for (int i = threadIdx.x; i < nb; i += blockDim.x)
-    if (hist[i] != 0.0) atomicAdd(wbar + i, hist[i]);
 }
 
 cudaError_t launch_blocked_adjoint(const GridDev& g, const BeamDev& b, const BeamletDev& bl, int S, const float* T,
                                    const float* tbar, const int* list_count, const int* list_v, double* wbar,
                                    int n_sm, int* flags, cudaStream_t st) {
-  const size_t smem = (size_t)bl.rows * bl.cols * sizeof(double);
-  if (smem > (48u << 10)) {
-    // per device and cheap: set it on every launch that needs it
-    cudaError_t e = cudaFuncSetAttribute(blocked_adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  blocked_adjoint_kernel<<<n_sm * 2, ADJ_THREADS, smem, st>>>(g, b, bl, S, T, tbar, list_count, list_v, wbar, flags);
+  blocked_adjoint_kernel<<<n_sm * 3, ADJ_THREADS, 0, st>>>(g, b, bl, S, T, tbar, list_count, list_v, wbar, flags);
   return cudaGetLastError();
 }
 
