@@ -16,11 +16,14 @@ namespace ch {
 #define SPEC_N2(X) X(3) X(4) X(5) X(6) X(8) X(9) X(10) X(12) X(15) X(16) X(18) X(20) X(24) X(27) X(32)
 
 // A CTA takes 16 lines: 16 N2 threads in the 16-point stages, 256 in the
-// N2-point ones.  CTAs per SM by registers (the N2-point stage holds 4 N2
-// values) and, along x, by shared memory.
+// N2-point ones.  r16n_ctas: CTAs per SM of the y and z passes, which stream and
+// gain from warps in flight until the N2-point stage spills.  Cone stage of 8
+// beams at 4, 3, 2, 1 CTAs (N2 up to 12, 16, 24, 32) / these / one more:
+// 96^3 197 / 186 / 210 us, 144^3 671 / 592 / 611, 160^3 925 / 842 / 871, 192^3
+// 1519 / 1423 / 1506, 201^3 3009 / 2583 / 3195.
 template <int N2>
 constexpr int r16n_threads() { return 16 * N2 > 256 ? 16 * N2 : 256; }
 template <int N2>
-constexpr int r16n_ctas() { return N2 <= 12 ? 4 : N2 <= 16 ? 3 : N2 <= 24 ? 2 : 1; }
+constexpr int r16n_ctas() { return N2 <= 12 ? 6 : N2 <= 16 ? 5 : N2 <= 20 ? 4 : N2 <= 24 ? 3 : 2; }
 
 }  // namespace ch

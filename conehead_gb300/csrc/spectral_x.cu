@@ -15,13 +15,17 @@ namespace ch {
 extern __shared__ float2 spec_sm[];
 
 // exchange and S^ block, and up to N2 = 24 a twiddle table (432 x 16 without
-// it leaves two CTAs per SM)
+// it leaves two CTAs per SM).  CTAs per SM: as many as shared memory and
+// spill-free registers allow; measured against one more and one fewer, cone
+// stage of 8 beams, fewer / this / more: 64^3 69.9 / 67.9 / 68 us, 144^3 715 /
+// 671 us / (no room), 160^3 924 / 971 us at 3 CTAs of N2 = 20.  Without the
+// staged S^ block (read through L2 in stage 2): 160^3 842 -> 1072-1184 us.
 template <int N2>
 constexpr bool x_table() { return N2 <= 24; }
 template <int N2>
 constexpr int x_smem() { return (2 * 16 * N2 * 16 + (x_table<N2>() ? 16 * N2 : 0)) * 8; }
 template <int N2>
-constexpr int x_ctas() { return N2 <= 12 ? 4 : N2 <= 16 ? 3 : N2 <= 24 ? 2 : 1; }
+constexpr int x_ctas() { return N2 <= 10 ? 5 : N2 <= 12 ? 4 : N2 <= 18 ? 3 : 2; }
 
 template <int N2>
 __global__ void __launch_bounds__(r16n_threads<N2>(), x_ctas<N2>()) spec_x_kernel(SpecLaunch P) {
