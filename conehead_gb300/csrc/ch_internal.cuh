@@ -265,6 +265,7 @@ struct SpecGrid {
   const float2* shat;      // S^ [Mx][My][Mz], 1/(Mx My Mz) folded in; [Mz][My][Mx] on the plane path
   int plane;               // the plane path (spec_plane_path): A = [Mz][lp] plane-major, no B
   int lp;                  // plane pitch of A on the plane path (nx ny rounded up to 32)
+  int after;               // the passes start while their predecessors end (launch_after)
 };
 struct SpecLaunch {
   SpecGrid g;
@@ -287,7 +288,7 @@ int spec_pass_lines_log2(int M, int Mz);
 std::vector<float2> spec_twiddles();      // every length (ascending), back to back
 size_t spec_twiddle_offset(int M);       // of exp(-2 pi i k / M); the quarter steps follow
 cudaError_t setup_spec_kernels();        // allow the kernels their dynamic shared memory
-void launch_spec_beams(const SpecLaunch& L, cudaStream_t st);
+void launch_spec_beams(SpecLaunch& L, cudaStream_t st);   // sets L.g.after
 // The plane path: periods of 256 along x and y (97 to 128 voxels).  z forward
 // into plane-major A[kz][x y], one cluster of two CTAs per (beam, kz) plane for
 // the y and x transforms, the S^ product and their inverses (the plane's
@@ -326,6 +327,66 @@ struct FusedRecords {
   PrologueBeam r[FUSED_MAX_BEAMS];
 };
 static_assert(sizeof(FusedRecords) <= 3968, "the records fit the smallest kernel parameter space");
+
+// ---------------------------------------------- programmatic launches --
+// A kernel launched with launch_after may start while its predecessor on the
+// stream finishes: it sets up what no earlier kernel writes, then waits for the
+// predecessor's memory (after_wait) before it reads or writes anything else.
+// Each such kernel lets its own successor start (after_trigger) when its CTAs
+// have started; the successor waits for its end all the same, so waits chain
+// through the stream.  The short kernels of a single beam's call spend a good
+// part of their time between launches.
+__device__ __forceinline__ void after_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void after_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+
+// A load of what an earlier kernel wrote, zero unless ok: an ordinary one (the
+// read-only path promises data that does not change while the kernel runs, and
+// the compiler may move it above the wait), predicated so that a thread's loads
+// stay one batch.  The compiler keeps them in place: issue them before the
+// barrier that publishes a table, not after.
+// KEEP: leave the line in L1 (the wider y and x passes, 1% at 160^3 and 192^3;
+// the others are 5% faster without, 96^3).
+template <bool KEEP = false>
+__device__ __forceinline__ float2 load_after(const float2* p, bool ok) {
+  float2 v;
+  if (KEEP)
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %3, 0;\n mov.f32 %0, 0f00000000;\n mov.f32 %1, 0f00000000;\n"
+        " @p ld.global.v2.f32 {%0, %1}, [%2];\n}"
+        : "=f"(v.x), "=f"(v.y)
+        : "l"(p), "r"((int)ok));
+  else
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %3, 0;\n mov.f32 %0, 0f00000000;\n mov.f32 %1, 0f00000000;\n"
+        " @p ld.global.L1::no_allocate.v2.f32 {%0, %1}, [%2];\n}"
+        : "=f"(v.x), "=f"(v.y)
+        : "l"(p), "r"((int)ok));
+  return v;
+}
+__device__ __forceinline__ float load_after(const float* p, bool ok) {
+  float v;
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %2, 0;\n mov.f32 %0, 0f00000000;\n"
+               " @p ld.global.L1::no_allocate.f32 %0, [%1];\n}"
+               : "=f"(v)
+               : "l"(p), "r"((int)ok));
+  return v;
+}
+
+// early = false: an ordinary launch.
+template <typename... P, typename... A>
+void launch_after(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = early ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, P(args)...);   // a failure is the caller's cudaGetLastError
+}
 
 // ------------------------------------------------------------ launchers --
 void launch_prologue_fused(const FusedRecords& recs, int n_beams, long long max_lines, int* flag_word, int epoch,

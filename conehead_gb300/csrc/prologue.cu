@@ -714,6 +714,8 @@ __global__ void __launch_bounds__(256) cull_batch_kernel(const PrologueBeam* __r
   __shared__ int n_kept;
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, l0 = blockIdx.x * lpc;
+  after_trigger();
+  after_wait();
   {
     const PrologueBeam& G = recs[blockIdx.y];
     if (l0 >= G.g.n[0] * G.g.n[1]) return;   // whole CTA
@@ -943,6 +945,8 @@ __global__ void __launch_bounds__(256, 3) terma_batch_kernel(const PrologueBeam*
   const int lane = threadIdx.x & 31;
   PrologueBeam& R = Rw[threadIdx.x >> 5];
   int cur = -1, beam = 0, base = 0, count = 0;
+  after_trigger();
+  after_wait();
   for (;;) {
     int c = 0;
     if (lane == 0) c = atomicAdd(work, 1);
@@ -983,6 +987,8 @@ __global__ void __launch_bounds__(256, 3) prologue_fused_kernel(const __grid_con
   const GridDev& g = R.g;
   const BeamDev& b = R.b;
   const int line = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  after_trigger();
+  after_wait();
   if (line >= g.n[0] * g.n[1]) return;   // whole warp
   const int x = line / g.n[1], y = line - x * g.n[1], nz = g.n[2];
   float pos[3] = {voxel_centre(g.origin[0], g.spacing[0], x), voxel_centre(g.origin[1], g.spacing[1], y), 0.0f};
@@ -1016,7 +1022,7 @@ __global__ void __launch_bounds__(256, 3) prologue_fused_kernel(const __grid_con
 
 void launch_prologue_fused(const FusedRecords& recs, int n_beams, long long max_lines, int* flag_word, int epoch,
                            cudaStream_t st) {
-  prologue_fused_kernel<<<dim3((unsigned)((max_lines + 7) / 8), n_beams), 256, 0, st>>>(recs, flag_word, epoch);
+  launch_after(true, prologue_fused_kernel, dim3((unsigned)((max_lines + 7) / 8), n_beams), 256, 0, st, recs, flag_word, epoch);
 }
 
 // ----------------------------------------------------- beamlet adjoint --
@@ -1283,12 +1289,13 @@ void launch_prologue_batch(const PrologueBeam* recs, int n_beams, long long max_
   // lines per CTA: enough CTAs for every SM's resident ones, at most 128 lines
   const long long per = max_lines * n_beams / ((long long)n_sm * 8);
   const int lpc = (int)std::min(128ll, std::max(16ll, per / 16 * 16));
-  cull_batch_kernel<<<dim3((unsigned)((max_lines + lpc - 1) / lpc), n_beams), threads, 0, st>>>(recs, lpc);
+  launch_after(true, cull_batch_kernel, dim3((unsigned)((max_lines + lpc - 1) / lpc), n_beams), threads, 0, st, recs, lpc);
   // persistent: at most the resident CTAs (3 per SM at 80 registers), fewer
   // for small batches; the warps share all beams' chunks
   const long long want = ((long long)n_beams * max_voxels + threads - 1) / threads;
   const long long cap = (long long)n_sm * std::min(ctas_per_sm, 3);
-  terma_batch_kernel<<<(unsigned)std::max(1ll, std::min(cap, want)), threads, 0, st>>>(recs, n_beams, flags, work);
+  launch_after(true, terma_batch_kernel, dim3((unsigned)std::max(1ll, std::min(cap, want))), threads, 0, st, recs, n_beams,
+               flags, work);
 }
 
 __global__ void init_scratch_kernel(int* aabb, int n_beams, int* counters) {

@@ -510,6 +510,7 @@ __device__ __forceinline__ void plane_load_row(const float2* Y, uint32_t peer, i
   }
 }
 
+template <bool AFTER>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PLANE_THREADS, 1) spec_plane_kernel(SpecLaunch P) {
   constexpr int H = SPEC_PLANE_M / 2;              // ky per CTA, and the largest nx
   float2* const Y = spec_sm;                         // [H][H], swizzled
@@ -539,12 +540,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PLANE_THREADS, 1) sp
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int y = j + 16 * q;
-      v[q] = (x < nx && y < ny) ? __ldg(plane + (size_t)x * ny + y) : make_float2(0.0f, 0.0f);
+      if (AFTER)
+        v[q] = load_after(plane + (size_t)x * ny + y, x < nx && y < ny);
+      else
+        v[q] = (x < nx && y < ny) ? __ldg(plane + (size_t)x * ny + y) : make_float2(0.0f, 0.0f);
     }
   };
   auto col_of = [&](int it) { return 2 * (PLANE_WARPS * it + warp) + c; };
 
   cluster_arrive_relaxed();
+  if (AFTER) {
+    after_trigger();
+    after_wait();   // S^ and the twiddles are older than any kernel of this call
+  }
   float2 pa[8];
   load_a(0, pa);
 
@@ -759,8 +767,8 @@ cudaError_t setup_spec_kernels() {
                         (const void*)spec_y_general_kernel<false>, (const void*)spec_y_general_kernel<true>,
                         (const void*)spec_x_general_kernel, (const void*)spec_full_general_kernel})
     if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, SPEC_SMEM);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(spec_plane_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SPEC_PLANE_SMEM);
+  for (const void* f : {(const void*)spec_plane_kernel<false>, (const void*)spec_plane_kernel<true>})
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, SPEC_PLANE_SMEM);
   return e;
 }
 
@@ -787,12 +795,23 @@ static void y_pass(const SpecLaunch& L, bool inverse, cudaStream_t st) {
     spec_y_general_kernel<false><<<g, SPEC_THREADS, SPEC_SMEM, st>>>(L);
 }
 
-void launch_spec_beams(const SpecLaunch& L, cudaStream_t st) {
+// The passes of a launch start while their predecessors end where they are
+// short: the work array A holds at most SPEC_AFTER_MAX values.  Cone stages
+// without / with, same kernels: one beam 40^3 24.8 / 16.4 us, 64^3 28.8 / 21.8,
+// 96^3 45 / 36, 160^3 131 / 118; 7 beams 64^3 61.7 / 48.8, 96^3 166 / 152, 128^3
+// (14.7 M) 297 / 297, 144^3 (20.9 M) 521 / 566, 192^3 1293 / 1404, one 192^3 (7.1
+// M) 233 / 239: a large pass
+// gains nothing and its successor's CTAs take its last wave's place.
+constexpr long long SPEC_AFTER_MAX = 6 << 20;
+
+void launch_spec_beams(SpecLaunch& L, cudaStream_t st) {
+  L.g.after = (long long)L.n_beams * L.g.n[0] * L.g.n[1] * L.g.M[2] <= SPEC_AFTER_MAX ? 1 : 0;
   z_pass(L, false, st);
   if (L.g.plane) {
     // clusters of two along x: consecutive clusters take the same kz plane of
     // consecutive beams
-    spec_plane_kernel<<<dim3(2 * L.n_beams, L.g.M[2]), PLANE_THREADS, SPEC_PLANE_SMEM, st>>>(L);
+    launch_after(L.g.after, L.g.after ? spec_plane_kernel<true> : spec_plane_kernel<false>,
+                 dim3(2 * L.n_beams, L.g.M[2]), PLANE_THREADS, SPEC_PLANE_SMEM, st, L);
   } else {
     y_pass(L, false, st);
     if (!launch_spec_x(L, st))

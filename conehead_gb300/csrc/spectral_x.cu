@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), x_ctas<N2>()) spec_x_kerne
   float2* const b = P.p[beam].b + off;
   const int nx = P.g.n[0];
   const int c = threadIdx.x & 15, h = threadIdx.x >> 4;   // h: n2 (stages 1, B) or k1 (stages 2, A)
+  after_trigger();
   {
     // S^ rows of the CTA's 16 lines: M x 128 bytes, 16 bytes per copy
     const float2* sh = P.g.shat + off;
@@ -50,19 +51,25 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), x_ctas<N2>()) spec_x_kerne
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(sh + (size_t)i * xs + cp));
     }
     asm volatile("cp.async.commit_group;\n" ::);
-    if (x_table<N2>())
-      for (int i = threadIdx.x; i < M; i += T) twb[i] = __ldg(P.g.tw[0] + i);
+  }
+  static_assert(M <= T, "one table entry per thread");
+  const float2 w_mine = x_table<N2>() ? __ldg(P.g.tw[0] + min((int)threadIdx.x, M - 1)) : make_float2(0.0f, 0.0f);
+  after_wait();   // S^ and the twiddles are older than any kernel of this call
+  float2 v[16];
+  if (threadIdx.x < 16 * N2) {
+#pragma unroll
+    for (int n1 = 0; n1 < 8; ++n1) {
+      const int x = N2 * n1 + h;
+      v[n1] = load_after<(N2 > 12)>(b + (size_t)x * xs + c, x < nx);
+    }
   }
   auto tw = [&](int i) { return x_table<N2>() ? twb[i] : __ldg(P.g.tw[0] + i); };
-  if (x_table<N2>()) __syncthreads();   // twiddle table
+  if (x_table<N2>()) {
+    if (threadIdx.x < M) twb[threadIdx.x] = w_mine;
+    __syncthreads();   // twiddle table
+  }
   if (threadIdx.x < 16 * N2) {
     // forward stage 1, thread (c, n2 = h): rows N2 n1 + n2, n1 < 8
-    float2 v[16];
-#pragma unroll
-    for (int n1 = 0; n1 < 16; ++n1) {
-      const int x = N2 * n1 + h;
-      v[n1] = (n1 < 8 && x < nx) ? __ldg(b + (size_t)x * xs + c) : make_float2(0.0f, 0.0f);
-    }
     dft16_half_in<false>(v);
     // X[m] of the DFT16 sits in v[4 (m mod 4) + m / 4]
 #pragma unroll
@@ -103,7 +110,6 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), x_ctas<N2>()) spec_x_kerne
   __syncthreads();
   if (threadIdx.x < 16 * N2) {
     // inverse stage B, thread (c, n2 = h): rows n2 + N2 n1
-    float2 v[16];
 #pragma unroll
     for (int q = 0; q < 16; ++q) v[q] = xb[(h * 16 + q) * 16 + c];
     dft16<true>(v);
@@ -176,7 +182,7 @@ bool launch_spec_x(const SpecLaunch& L, cudaStream_t st) {
   switch (L.g.M[0]) {
 #define X_CASE(N2)                                                                  \
   case 16 * N2:                                                                     \
-    spec_x_kernel<N2><<<grid, r16n_threads<N2>(), x_smem<N2>(), st>>>(L);           \
+    launch_after(L.g.after, spec_x_kernel<N2>, grid, r16n_threads<N2>(), x_smem<N2>(), st, L); \
     return true;
     SPEC_N2(X_CASE)
 #undef X_CASE

@@ -33,17 +33,29 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), r16n_ctas<N2>()) spec_y_ke
   const float2* const src = (INV ? bm.b + (size_t)x * M * L : bm.a + (size_t)x * ny * L) + kz0;
   float2* const dst = (INV ? bm.a + (size_t)x * ny * L : bm.b + (size_t)x * M * L) + kz0;
   const int c = threadIdx.x & 15, h = threadIdx.x >> 4;   // h: n2 (stages 1, B) or k1 (stages 2, A)
-  for (int i = threadIdx.x; i < M; i += T) twb[i] = __ldg(P.g.tw[1] + i);
+  static_assert(M <= T, "one table entry per thread");
+  after_trigger();
+  const float2 w_mine = __ldg(P.g.tw[1] + min((int)threadIdx.x, M - 1));
+  after_wait();
+  // the inputs are in flight while the table is published
+  float2 v[16], a[N2];
+  if (!INV) {
+    if (threadIdx.x < 16 * N2) {
+#pragma unroll
+      for (int n1 = 0; n1 < 8; ++n1) {
+        const int y = N2 * n1 + h;
+        v[n1] = load_after<(N2 > 12)>(src + (size_t)y * L + c, y < ny);
+      }
+    }
+  } else if (threadIdx.x < 256) {
+#pragma unroll
+    for (int k2 = 0; k2 < N2; ++k2) a[k2] = load_after<(N2 > 12)>(src + (size_t)(h + 16 * k2) * L + c, true);
+  }
+  if (threadIdx.x < M) twb[threadIdx.x] = w_mine;
   __syncthreads();   // twiddle table
   if (!INV) {
     if (threadIdx.x < 16 * N2) {
       // stage 1, thread (c, n2 = h)
-      float2 v[16];
-#pragma unroll
-      for (int n1 = 0; n1 < 16; ++n1) {
-        const int y = N2 * n1 + h;
-        v[n1] = (n1 < 8 && y < ny) ? __ldg(src + (size_t)y * L + c) : make_float2(0.0f, 0.0f);
-      }
       dft16_half_in<false>(v);
 #pragma unroll
       for (int m = 0; m < 16; ++m) {
@@ -55,7 +67,6 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), r16n_ctas<N2>()) spec_y_ke
     __syncthreads();
     if (threadIdx.x < 256) {
       // stage 2, thread (c, k1 = h)
-      float2 a[N2];
 #pragma unroll
       for (int n2 = 0; n2 < N2; ++n2) a[n2] = xb[(h * N2 + n2) * 16 + c];
       Dft<false, N2>::run(a);
@@ -65,9 +76,6 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), r16n_ctas<N2>()) spec_y_ke
   } else {
     if (threadIdx.x < 256) {
       // stage A, thread (c, k1 = h)
-      float2 a[N2];
-#pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2) a[k2] = __ldg(src + (size_t)(h + 16 * k2) * L + c);
       Dft<true, N2>::run(a);
 #pragma unroll
       for (int n2 = 0; n2 < N2; ++n2) {
@@ -82,7 +90,6 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), r16n_ctas<N2>()) spec_y_ke
     __syncthreads();
     if (threadIdx.x < 16 * N2) {
       // stage B, thread (c, n2 = h)
-      float2 v[16];
 #pragma unroll
       for (int q = 0; q < 16; ++q) v[q] = xb[(h * 16 + q) * 16 + c];
       dft16<true>(v);
@@ -119,9 +126,9 @@ bool launch_spec_y(const SpecLaunch& L, bool inverse, cudaStream_t st) {
 #define Y_CASE(N2)                                                                     \
   case 16 * N2:                                                                        \
     if (inverse)                                                                       \
-      spec_y_kernel<true, N2><<<grid, r16n_threads<N2>(), y_smem<N2>(), st>>>(L);      \
+      launch_after(L.g.after, spec_y_kernel<true, N2>, grid, r16n_threads<N2>(), y_smem<N2>(), st, L); \
     else                                                                               \
-      spec_y_kernel<false, N2><<<grid, r16n_threads<N2>(), y_smem<N2>(), st>>>(L);     \
+      launch_after(L.g.after, spec_y_kernel<false, N2>, grid, r16n_threads<N2>(), y_smem<N2>(), st, L); \
     return true;
     SPEC_N2(Y_CASE)
 #undef Y_CASE

@@ -54,16 +54,18 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), r16n_ctas<N2>()) spec_z_fo
   const SpecBeam& bm = P.p[blockIdx.y];
   const int nl = P.g.n[0] * P.g.n[1], nz = P.g.n[2];
   const int l0 = blockIdx.x * 16;
+  after_trigger();
+  // stage-1 twiddles exp(-2 pi i n2 (4 m + 1) / (4 L)) at m N2 + n2
+  for (int i = threadIdx.x; i < L; i += T) twb[i] = __ldg(P.g.tq + (i % N2) * (4 * (i / N2) + 1));
+  after_wait();
   // lines that may hold TERMA (the others are zero and are not read)
   __shared__ unsigned char zf[16];
   bool mine = false;
   if (threadIdx.x < 16) {
     const int l = l0 + threadIdx.x;
-    mine = l < nl && (!bm.l || __ldg(bm.l + l) != 0);
+    mine = l < nl && (!bm.l || bm.l[l] != 0);
     zf[threadIdx.x] = mine;
   }
-  // stage-1 twiddles exp(-2 pi i n2 (4 m + 1) / (4 L)) at m N2 + n2
-  for (int i = threadIdx.x; i < L; i += T) twb[i] = __ldg(P.g.tq + (i % N2) * (4 * (i / N2) + 1));
   if (!__syncthreads_or(mine)) {
     // no TERMA on these lines: zeros, two values per 16-byte store
     if constexpr (PLANE) {
@@ -86,9 +88,10 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), r16n_ctas<N2>()) spec_z_fo
 #pragma unroll
     for (int n1 = 0; n1 < 16; ++n1) {
       const int z = N2 * n1 + n2;
-      const float x = (live && z < nz) ? __ldg(t + z) : 0.0f;
-      v[n1] = make_float2(x * W.c[n1], -x * W.s[n1]);
+      v[n1].x = load_after(t + z, live && z < nz);
     }
+#pragma unroll
+    for (int n1 = 0; n1 < 16; ++n1) v[n1] = make_float2(v[n1].x * W.c[n1], -v[n1].x * W.s[n1]);
     dft16<false>(v);
     // X[m] of the DFT16 sits in v[4 (m mod 4) + m / 4]
 #pragma unroll
@@ -121,8 +124,12 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), r16n_ctas<N2>()) spec_z_in
   const SpecBeam& bm = P.p[blockIdx.y];
   const int nl = P.g.n[0] * P.g.n[1], nz = P.g.n[2];
   const int l0 = blockIdx.x * 16;
-  // stage-A twiddles at 16 n2 + k1
-  for (int i = threadIdx.x; i < L; i += T) twb[i] = __ldg(P.g.tq + (i >> 4) * (4 * (i & 15) + 1));
+  after_trigger();
+  // stage-A twiddles at 16 n2 + k1, one per thread
+  static_assert(L <= T, "one table entry per thread");
+  const int i_mine = min((int)threadIdx.x, L - 1);
+  const float2 w_mine = __ldg(P.g.tq + (i_mine >> 4) * (4 * (i_mine & 15) + 1));
+  after_wait();
   const int lo = threadIdx.x & 15, hi = threadIdx.x >> 4;
   float2 a[N2];
   if (threadIdx.x < 256) {
@@ -130,9 +137,10 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), r16n_ctas<N2>()) spec_z_in
 #pragma unroll
     for (int k2 = 0; k2 < N2; ++k2) {
       const int k = k1 + 16 * k2;
-      a[k2] = l < nl ? __ldg(bm.a + (PLANE ? (size_t)k * P.g.lp + l : (size_t)l * L + k)) : make_float2(0.0f, 0.0f);
+      a[k2] = load_after(bm.a + (PLANE ? (size_t)k * P.g.lp + l : (size_t)l * L + k), l < nl);
     }
   }
+  if (threadIdx.x < L) twb[threadIdx.x] = w_mine;
   __syncthreads();   // twiddle table
   if (threadIdx.x < 256) {
     const int k1 = PLANE ? hi : lo, c = PLANE ? lo : hi;
@@ -190,13 +198,13 @@ bool launch_spec_z(const SpecLaunch& L, bool inverse, cudaStream_t st) {
 #define Z_CASE(N2)                                                                                          \
   case 16 * N2:                                                                                             \
     if (L.g.plane && !inverse)                                                                              \
-      spec_z_forward_kernel<N2, true><<<grid, r16n_threads<N2>(), z_smem<N2, true>(), st>>>(L);             \
+      launch_after(L.g.after, spec_z_forward_kernel<N2, true>, grid, r16n_threads<N2>(), z_smem<N2, true>(), st, L); \
     else if (L.g.plane)                                                                                     \
-      spec_z_inverse_kernel<N2, true><<<grid, r16n_threads<N2>(), z_smem<N2, true>(), st>>>(L);             \
+      launch_after(L.g.after, spec_z_inverse_kernel<N2, true>, grid, r16n_threads<N2>(), z_smem<N2, true>(), st, L); \
     else if (!inverse)                                                                                      \
-      spec_z_forward_kernel<N2, false><<<grid, r16n_threads<N2>(), z_smem<N2, false>(), st>>>(L);           \
+      launch_after(L.g.after, spec_z_forward_kernel<N2, false>, grid, r16n_threads<N2>(), z_smem<N2, false>(), st, L); \
     else                                                                                                    \
-      spec_z_inverse_kernel<N2, false><<<grid, r16n_threads<N2>(), z_smem<N2, false>(), st>>>(L);           \
+      launch_after(L.g.after, spec_z_inverse_kernel<N2, false>, grid, r16n_threads<N2>(), z_smem<N2, false>(), st, L); \
     return true;
     SPEC_N2(Z_CASE)
 #undef Z_CASE
