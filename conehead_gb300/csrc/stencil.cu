@@ -209,17 +209,12 @@ __global__ void __launch_bounds__(128) scatter_kernel(const float* __restrict__ 
   }
 }
 
-// kernel_index without float64: the float64 form floors 100 t - 5 exactly
-// (31 significand bits), so the float32 product p and its residual e decide
-// it -- floor(p + e) = floor(p) unless p is an integer and e < 0.  (Within
-// 2^-51 below zero the float64 form rounds to -5.)  NaN and values whose int64
-// conversion saturates below give 0, as there.
-__device__ __forceinline__ int kernel_index_f32(float t) {
-  const float p = __fmul_rn(t, 100.0f), e = __fmaf_rn(t, 100.0f, -p);
-  float f = floorf(p + 4.44089210e-16f);
-  if (f == p && e < 0.0f) f -= 1.0f;
-  if (!(p > -9.223372036854775808e18f)) return 0;
-  return (int)fminf(fabsf(f - 5.0f), 5995.0f);
+// kernel_index without float64 for t >= 0, p = 100 t rounded down: the float64
+// form floors 100 t - 5 exactly (31 significand bits); the product rounded down
+// has the same floor, which an addition rounding down to a step of 1 leaves in
+// the low mantissa bits.
+__device__ __forceinline__ int kernel_index_f32(float p) {
+  return min(abs(__float_as_int(__fadd_rd(fminf(p, 6100.0f), 12582912.0f)) - (0x4b400000 + 5)), 5995);
 }
 
 // K as pairs of float32, hi + lo: 48 significand bits
@@ -252,26 +247,36 @@ __device__ __forceinline__ float pair_diff(float2 k1, float2 k0) {
 // of the prologue (swap_xy).  Each unique walk carries its multiplicity.
 //
 // A warp takes 32 entries of the prologue's voxel list (one per lane, most of
-// them neighbours along z) and RADIO_GROUP walks: its lanes read the same taps,
-// and a step's adds fall in one or two 128-byte lines of the dose.  Steps go
-// RADIO_UNROLL at a time so that their density reads, and then their table
-// reads, are in flight together.  One thread per grid voxel walking all 576
+// them neighbours along z) and RADIO_GROUP walks: its lanes step through the same
+// taps, and a step's adds fall in one or two 128-byte lines of the dose.  What
+// a tap means for every lane -- its linear offsets, its segment, how far it is
+// from the start -- is worked out by one lane for each of 32 taps and handed
+// round by shuffles; the offsets' distances against the voxel's room to the
+// grid's faces are one subtraction of packed fields (grids of up to 512 voxels
+// per axis, PACKED).  Steps go RADIO_UNROLL at a time so that their density reads,
+// and then their table reads, are in flight together.
+//
+// 48^3 at 0.4 cm with a 5 x 5 cm field: one thread per grid voxel walking all 576
 // cones left 3 warps in 4 without a source and the others with 40 thousand
-// dependent steps, each with seven float64 instructions (two lanes per clock
-// and SM here): 48^3 at 0.4 cm with a 5 x 5 cm field 14830 -> 1350 us.
+// dependent steps, each with seven float64 instructions (two lanes per clock and
+// SM here), 14830 us; warps with every lane working out every tap, 104
+// instructions a step, 1350 us; this 890 us, still issue bound.
 constexpr int RADIO_GROUP = 8, RADIO_UNROLL = 4;
+template <bool PACKED>
 __global__ void __launch_bounds__(256) scatter_radiological_kernel(
     const float* __restrict__ T, const float* __restrict__ rho, int n0, int n1, int n2, int zp, int swap_xy,
     int n_dirs, const int* __restrict__ tap_base, const int* __restrict__ tap_len, const short4* __restrict__ offs,
     const float* __restrict__ tvals, const int* __restrict__ walk_row, const int* __restrict__ walk_mult,
     const float2* __restrict__ K2, int n_r, const int* __restrict__ list_count, const int* __restrict__ list_v,
     float* __restrict__ dose) {
+  const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   const int count = *list_count, chunks = (count + 31) >> 5;
   const int groups = (n_dirs + RADIO_GROUP - 1) / RADIO_GROUP;
   // density index of (x, y, z): steps along x and y as the reference reads them
   const int rx = swap_xy ? n2 : n1 * n2, ry = swap_xy ? n0 * n2 : n2;
+  constexpr int OK = (1 << 9) | (1 << 19) | (1 << 29);   // a field of 512 + room - distance keeps this bit
   const long long items = (long long)chunks * groups;
   for (long long item = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; item < items; item += warps) {
     const int gr = (int)(item / chunks), chunk = (int)(item - (long long)gr * chunks);
@@ -287,52 +292,96 @@ __global__ void __launch_bounds__(256) scatter_radiological_kernel(
       Tv = T[((size_t)x * n1 + y) * zp + z];
     }
     const bool source = Tv != 0.0f;
-    if (!__any_sync(0xffffffffu, source)) continue;
-    const int dv = (x * n1 + y) * n2 + z, rv = x * rx + y * ry + z;
+    if (!__any_sync(full, source)) continue;
+    float* const dv = dose + (x * n1 + y) * n2 + z;
+    const float* const rv = rho + (x * rx + y * ry + z);
     const int u1 = min(n_dirs, (gr + 1) * RADIO_GROUP);
     for (int u = gr * RADIO_GROUP; u < u1; ++u) {
       const int b = __ldg(tap_base + u), L = __ldg(tap_len + u);
+      if (L <= 0) continue;
       const float2* Kj = K2 + (size_t)__ldg(walk_row + u) * n_r;
       const float mult = (float)__ldg(walk_mult + u);
-      float rad = 0.0f, tprev = 0.0f;
+      // every axis steps one way: the last tap has its sign
+      const short4 end = __ldg(offs + b + L - 1);
+      const int room = ((end.x < 0 ? x : n0 - 1 - x) + 512) | ((end.y < 0 ? y : n1 - 1 - y) + 512) << 10 |
+                       ((end.z < 0 ? z : n2 - 1 - z) + 512) << 20;
+      float rad = 0.0f, tlast = 0.0f;
       float2 kp = make_float2(0.0f, 0.0f);
       int prev = -1;
       bool alive = source, ended = false;
-      for (int m0 = 0; m0 < L && __any_sync(0xffffffffu, alive); m0 += RADIO_UNROLL) {
-        float rh[RADIO_UNROLL], tv[RADIO_UNROLL];
-        int at[RADIO_UNROLL], ki[RADIO_UNROLL];
-        bool in[RADIO_UNROLL];
+      for (int m0 = 0; m0 < L; m0 += 32) {
+        // tap m0 + lane
+        const int m = min(m0 + lane, L - 1);
+        const short4 o = __ldg(offs + b + m);
+        const float t = __ldg(tvals + b + m);
+        float t_before = __shfl_up_sync(full, t, 1);
+        if (lane == 0) t_before = tlast;
+        tlast = __shfl_sync(full, t, 31);
+        const float seg = fsub(t, t_before);
+        const int at = (o.x * n1 + o.y) * n2 + o.z, rat = o.x * rx + o.y * ry + o.z;
+        // beyond every room past the last tap
+        const int far = PACKED ? (m0 + lane < L ? min(abs(o.x), 512) : 512) | min(abs(o.y), 512) << 10 |
+                                     min(abs(o.z), 512) << 20
+                               : (int)(unsigned short)(m0 + lane < L ? o.x : 8192) | (int)o.y << 16;
+        const int n = min(32, L - m0);
+        for (int s0 = 0; s0 < n && __any_sync(full, alive); s0 += RADIO_UNROLL) {
+          float rh[RADIO_UNROLL], sg[RADIO_UNROLL];
+          int to[RADIO_UNROLL], ki[RADIO_UNROLL];
+          bool in[RADIO_UNROLL];
 #pragma unroll
-        for (int q = 0; q < RADIO_UNROLL; ++q) {
-          const int m = min(m0 + q, L - 1);
-          const short4 o = __ldg(offs + b + m);
-          tv[q] = __ldg(tvals + b + m);
-          alive = alive && m0 + q < L && (unsigned)(x + o.x) < (unsigned)n0 && (unsigned)(y + o.y) < (unsigned)n1 &&
-                  (unsigned)(z + o.z) < (unsigned)n2;
-          in[q] = alive;
-          at[q] = (o.x * n1 + o.y) * n2 + o.z;
-          rh[q] = alive ? __ldg(rho + (rv + o.x * rx + o.y * ry + o.z)) : 0.0f;
-        }
-        float2 kv[RADIO_UNROLL];
-#pragma unroll
-        for (int q = 0; q < RADIO_UNROLL; ++q) {
-          rad = fadd(rad, fmul(rh[q], fsub(tv[q], tprev)));
-          tprev = tv[q];
-          ki[q] = kernel_index_f32(rad);
-          kv[q] = in[q] ? __ldg(Kj + ki[q]) : make_float2(0.0f, 0.0f);
-        }
-#pragma unroll
-        for (int q = 0; q < RADIO_UNROLL; ++q) {
-          // saturated twice: the walk has ended, whatever its next steps read
-          ended = ended || (prev == 5995 && ki[q] == 5995);
-          if (in[q] && !ended) {
-            const float dk = prev < 0 ? fadd(kv[q].x, kv[q].y) : pair_diff(kv[q], kp);
-            atomicAdd(dose + (dv + at[q]), Tv * __fmul_rn(dk, mult));
+          for (int q = 0; q < RADIO_UNROLL; ++q) {
+            const int s = s0 + q;
+            const int f = __shfl_sync(full, far, s), ro = __shfl_sync(full, rat, s);
+            to[q] = __shfl_sync(full, at, s);
+            sg[q] = __shfl_sync(full, seg, s);
+            if (PACKED) {
+              alive = alive && ((room - f) & OK) == OK;
+            } else {
+              const int oz = __shfl_sync(full, (int)o.z, s);
+              alive = alive && (unsigned)(x + (int)(short)f) < (unsigned)n0 && (unsigned)(y + (f >> 16)) < (unsigned)n1 &&
+                      (unsigned)(z + oz) < (unsigned)n2;
+            }
+            in[q] = alive;
+            rh[q] = alive ? __ldg(rv + ro) : 0.0f;
           }
-          prev = ki[q];
-          kp = kv[q];
+          float2 kv[RADIO_UNROLL];
+          bool plain = true;     // no negative or undefined distance
+          int top = 0;
+#pragma unroll
+          for (int q = 0; q < RADIO_UNROLL; ++q) {
+            rad = fadd(rad, fmul(rh[q], sg[q]));
+            rh[q] = rad;
+            const float p = __fmul_rd(rad, 100.0f);
+            plain = plain && p >= 0.0f;
+            ki[q] = kernel_index_f32(p);
+            top = max(top, ki[q]);
+          }
+          if (!plain) {          // the float64 form
+            top = 5995;
+#pragma unroll
+            for (int q = 0; q < RADIO_UNROLL; ++q) ki[q] = kernel_index(rh[q]);
+          }
+#pragma unroll
+          for (int q = 0; q < RADIO_UNROLL; ++q) kv[q] = in[q] ? __ldg(Kj + ki[q]) : make_float2(0.0f, 0.0f);
+          if (top == 5995) {
+            // twice at the table's end: the walk has ended, whatever its next steps read
+#pragma unroll
+            for (int q = 0; q < RADIO_UNROLL; ++q) {
+              ended = ended || (prev == 5995 && ki[q] == 5995);
+              in[q] = in[q] && !ended;
+              prev = ki[q];
+            }
+          }
+          prev = ki[RADIO_UNROLL - 1];
+#pragma unroll
+          for (int q = 0; q < RADIO_UNROLL; ++q) {
+            // (the first tap's difference is to a pair of zeros)
+            if (in[q]) atomicAdd(dv + to[q], Tv * __fmul_rn(pair_diff(kv[q], kp), mult));
+            kp = kv[q];
+          }
+          alive = alive && !ended;
         }
-        alive = alive && !ended;
+        if (!__any_sync(full, alive)) break;
       }
     }
   }
@@ -342,9 +391,10 @@ void launch_scatter_radiological(const float* T, const float* rho, const int* n,
                                  const int* tap_base, const int* tap_len, const short4* offs, const float* tvals,
                                  const int* walk_row, const int* walk_mult, const float2* K2, int n_r,
                                  const int* list_count, const int* list_v, int n_sm, float* dose, cudaStream_t st) {
-  scatter_radiological_kernel<<<n_sm * 6, 256, 0, st>>>(T, rho, n[0], n[1], n[2], zp, swap_xy, n_dirs, tap_base,
-                                                        tap_len, offs, tvals, walk_row, walk_mult, K2, n_r,
-                                                        list_count, list_v, dose);
+  const bool packed = n[0] <= 512 && n[1] <= 512 && n[2] <= 512;
+  const auto kernel = packed ? scatter_radiological_kernel<true> : scatter_radiological_kernel<false>;
+  kernel<<<n_sm * 6, 256, 0, st>>>(T, rho, n[0], n[1], n[2], zp, swap_xy, n_dirs, tap_base, tap_len, offs, tvals,
+                                   walk_row, walk_mult, K2, n_r, list_count, list_v, dose);
 }
 
 void launch_scatter(const float* T, const int* n, int zp, int n_dirs, const int* tap_base, const int* tap_len,
