@@ -199,11 +199,10 @@ class MLCField:
         m.n_pairs = len(self.row0)
         m.map_rows, m.map_cols = self.rows, MAP_COLS
         m.open_r0, m.open_r1, m.open_c0, m.open_c1 = self.window
-        for n in range(m.n_pairs):
-            m.row0[n], m.rows[n] = int(self.row0[n]), int(self.rows_of[n])
-            m.a_end[n], m.b_start[n] = int(self.a_end[n]), int(self.b_start[n])
-        for k, v in enumerate(self.tip_ramp()):
-            m.tip[k] = float(v)
+        n = m.n_pairs
+        m.row0[:n], m.rows[:n] = self.row0.tolist(), self.rows_of.tolist()
+        m.a_end[:n], m.b_start[:n] = self.a_end.tolist(), self.b_start.tolist()
+        m.tip[:] = self.tip_ramp().tolist()
         return m
 
 

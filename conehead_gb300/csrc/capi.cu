@@ -128,6 +128,7 @@ struct ch_plan {
   int live_batches = 0;      // captured batches reading this plan's stencils
   long long wait_limit = 0;  // gather pipeline waits (try_wait iterations); 0 = MBAR_LIMIT
   int withhold = 0;          // test hook of the expired-wait path (ch_plan_set_wait_limit)
+  int* h_flags = nullptr;    // pinned copy of the counters (ch_plan_sync, ch_batch_sync)
   int epoch = 0;             // of the last call with the one-launch prologue
   bool flags_by_epoch = false;   // the last call reports failures in counters[6] == epoch, not in counters[1]
   int reweights = 0;         // spectrum switches served by reweighting the stencils
@@ -159,6 +160,7 @@ struct ch_plan {
   bool rec_pending[2] = {false, false};
   int rec_next = 0;
   ~ch_plan() {
+    if (h_flags) cudaFreeHost(h_flags);
     for (int i = 0; i < 2; ++i)
       if (rec_pending[i] && ev_rec[i]) cudaEventSynchronize(ev_rec[i]);
     spec.clear();
@@ -1932,6 +1934,22 @@ ch_status ch_dose_adjoint(ch_plan* P, const ch_grid* grid, const float* rho, int
   return CH_OK;
 }
 
+// Waits for `stream` and reports what its kernels left in `counters`: one copy
+// behind them into pinned memory and one wait (a wait and then a blocking copy
+// were two round trips).
+namespace {
+ch_status read_flags(ch_plan* P, const void* counters, cudaStream_t s, bool by_epoch) {
+  if (!P->h_flags) CH_CUDA(cudaMallocHost(&P->h_flags, 8 * sizeof(int)));
+  CH_CUDA(cudaMemcpyAsync(P->h_flags, counters, 8 * sizeof(int), cudaMemcpyDeviceToHost, s));
+  CH_CUDA(cudaStreamSynchronize(s));
+  const int* c = P->h_flags;
+  const int flags = by_epoch ? (c[6] == P->epoch ? FLAG_PARALLEL_RAY : 0) : c[1];
+  if (flags & FLAG_TIMEOUT) return fail(CH_ERR_TIMEOUT, "a bounded device wait expired in the cone stage");
+  if (flags & FLAG_PARALLEL_RAY) return fail(CH_ERR_PARALLEL_RAY, "no intersection or line is within plane");
+  return CH_OK;
+}
+}  // namespace
+
 // ------------------------------------------------------- captured batch --
 struct ch_batch {
   ch_plan* P = nullptr;
@@ -2020,12 +2038,7 @@ ch_status ch_batch_launch(ch_batch* bt, void* stream) {
 ch_status ch_batch_sync(ch_batch* bt, void* stream) {
   if (!bt) return fail(CH_ERR_INVALID_ARG, "batch is NULL");
   CH_CUDA(cudaSetDevice(bt->P->device));
-  CH_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-  int c[2];
-  CH_CUDA(cudaMemcpy(c, bt->counters.p, sizeof(c), cudaMemcpyDeviceToHost));
-  if (c[1] & FLAG_TIMEOUT) return fail(CH_ERR_TIMEOUT, "a bounded device wait expired in the cone stage");
-  if (c[1] & FLAG_PARALLEL_RAY) return fail(CH_ERR_PARALLEL_RAY, "no intersection or line is within plane");
-  return CH_OK;
+  return read_flags(bt->P, bt->counters.p, (cudaStream_t)stream, false);
 }
 
 void ch_batch_destroy(ch_batch* bt) {
@@ -2179,14 +2192,11 @@ ch_status ch_plan_set_wait_limit(ch_plan* P, long long iterations, int withhold)
 ch_status ch_plan_sync(ch_plan* P, void* stream) {
   if (!P) return fail(CH_ERR_INVALID_ARG, "plan is NULL");
   CH_CUDA(cudaSetDevice(P->device));
-  CH_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-  if (!P->counters.p) return CH_OK;
-  int c[8];
-  CH_CUDA(cudaMemcpy(c, P->counters.p, sizeof(c), cudaMemcpyDeviceToHost));
-  const int flags = P->flags_by_epoch ? (c[6] == P->epoch ? FLAG_PARALLEL_RAY : 0) : c[1];
-  if (flags & FLAG_TIMEOUT) return fail(CH_ERR_TIMEOUT, "a bounded device wait expired in the cone stage");
-  if (flags & FLAG_PARALLEL_RAY) return fail(CH_ERR_PARALLEL_RAY, "no intersection or line is within plane");
-  return CH_OK;
+  if (!P->counters.p) {
+    CH_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+    return CH_OK;
+  }
+  return read_flags(P, P->counters.p, (cudaStream_t)stream, P->flags_by_epoch);
 }
 
 ch_status ch_plan_stats(ch_plan* P, ch_stats* out) {
