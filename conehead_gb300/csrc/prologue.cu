@@ -254,7 +254,10 @@ __device__ __forceinline__ bool lattice_centre(const BeamDev& b, const float* po
   return !b.wraps || (c.u - c.mu > -1999.0f && c.w - c.mw > -1999.0f);
 }
 
-// Calls f(ix, iy, iz, u, w) for every sub-sample in the reference's order.
+// Calls f(ix, iy, iz, u, w) for every sub-sample in the reference's order.  Rolled:
+// three copies of a map lookup along z outgrew the instruction cache (nine MLC
+// beams, prologue 1.23 -> 1.05 ms with five steps of the walk below instead of
+// eight).
 template <class F>
 __device__ __forceinline__ void for_samples(const BeamDev& b, const float* off, int S, const Centre& c, F f) {
   const float K = 100.0f * b.a_K, c0 = 100.0f * b.a_c0, c2 = 100.0f * b.a_c2;
@@ -267,7 +270,7 @@ __device__ __forceinline__ void for_samples(const BeamDev& b, const float* off, 
     for (int iy = 0; iy < S; ++iy) {
       const float ry = off[1] * ((float)iy - mid);
       const float ny = nx - b.vyf[1] * ry, x0y = x0x - b.m0f[1] * ry, x2y = x2x - b.m2f[1] * ry;
-#pragma unroll 3
+#pragma unroll 1
       for (int iz = 0; iz < S; ++iz) {
         const float rz = off[2] * ((float)iz - mid);
         const float si = __fdividef(K, ny - b.vyf[2] * rz);
@@ -514,9 +517,9 @@ __device__ __forceinline__ double blocked_fraction(const BeamDev& b, const GridD
 // step along different axes, so three short branches cost every step all
 // three paths (20 of 32 lanes active; TERMA of 32 beams at 128^3 638 -> 509 us,
 // 547 -> 396 M warp instructions).  Also tried at 3 CTAs per SM: 4, 6 and 8
-// steps with the next group's loads issued before this one's sums, 12 steps,
+// steps with the next group's loads issued before this one's sums, 8 and 12 steps,
 // and 64 registers (4 CTAs): all within 2%.
-constexpr int DDA_UNROLL = 8;
+constexpr int DDA_UNROLL = 5;
 
 __device__ float radiological_depth(const float* __restrict__ rho, const GridDev& g, int x, int y, int z,
                                     const float* rd) {
