@@ -265,6 +265,7 @@ struct SpecGrid {
   const float2* shat;      // S^ [Mx][My][Mz], 1/(Mx My Mz) folded in; [Mz][My][Mx] on the plane path
   int plane;               // the plane path (spec_plane_path): A = [Mz][lp] plane-major, no B
   int lp;                  // plane pitch of A on the plane path (nx ny rounded up to 32)
+  int skip;                // rows of A without TERMA are not written: their reader goes by the line flags
   int after;               // the passes start while their predecessors end (launch_after)
 };
 struct SpecLaunch {

@@ -805,6 +805,11 @@ static void y_pass(const SpecLaunch& L, bool inverse, cudaStream_t st) {
 constexpr long long SPEC_AFTER_MAX = 6 << 20;
 
 void launch_spec_beams(SpecLaunch& L, cudaStream_t st) {
+  // rows of A without TERMA are neither written nor read where the y pass goes
+  // by the line flags (the kernels of lengths to 512): cone stage of 4 beams at 144^3 308 -> 298 us, 7 at 192^3
+  // 1282 -> 1252.  Not on the plane path, where the flags' latency (one CTA per
+  // SM) costs more than the rows: 32 beams at 128^3 1260 -> 1362.
+  L.g.skip = !L.g.plane && std::max(L.g.M[1], L.g.M[2]) <= 512;
   L.g.after = (long long)L.n_beams * L.g.n[0] * L.g.n[1] * L.g.M[2] <= SPEC_AFTER_MAX ? 1 : 0;
   z_pass(L, false, st);
   if (L.g.plane) {

@@ -10,6 +10,8 @@
 //       exp(+2 pi i n2 k1 / M), out to shared memory row 16 n2 + k1;
 //     stage B, thread (c, n2): 16-point DFT over k1 -> rows n2 + N2 n1,
 //       n1 < 8, written where < ny.
+// Rows of A whose line holds no TERMA are zero: the z pass does not write them and
+// the forward pass does not read them (launch_spec_beams has the figures).
 // A row of 16 lines is 128 bytes, one half-warp access: no swizzle is needed.
 
 #include "spectral_16n.cuh"
@@ -37,6 +39,7 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), r16n_ctas<N2>()) spec_y_ke
   after_trigger();
   const float2 w_mine = __ldg(P.g.tw[1] + min((int)threadIdx.x, M - 1));
   after_wait();
+  const unsigned char* const lines = P.g.skip && bm.l ? bm.l + x * ny : nullptr;
   // the inputs are in flight while the table is published
   float2 v[16], a[N2];
   if (!INV) {
@@ -44,7 +47,7 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), r16n_ctas<N2>()) spec_y_ke
 #pragma unroll
       for (int n1 = 0; n1 < 8; ++n1) {
         const int y = N2 * n1 + h;
-        v[n1] = load_after<(N2 > 12)>(src + (size_t)y * L + c, y < ny);
+        v[n1] = load_after<(N2 > 12)>(src + (size_t)y * L + c, y < ny && (!lines || lines[y] != 0));
       }
     }
   } else if (threadIdx.x < 256) {

@@ -67,6 +67,7 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), r16n_ctas<N2>()) spec_z_fo
     zf[threadIdx.x] = mine;
   }
   if (!__syncthreads_or(mine)) {
+    if (P.g.skip) return;
     // no TERMA on these lines: zeros, two values per 16-byte store
     if constexpr (PLANE) {
       for (int e = threadIdx.x; e < L * 8; e += T)
