@@ -1291,8 +1291,9 @@ ch_status enqueue_batch(ch_plan* P, const BatchPlan& B, const Scratch& S, const 
       const BeamJob& J = B.jobs[i];
       int all = 0;
       const Inter in = make_inter(inter, all);
+      // the cone stages here read no list: with all voxels none is made
       launch_prologue(J.rho, J.g, J.b, J.s, S.T + J.t_off, in, all, S.aabb + 8 * i, !B.spectral,
-                      S.list_v + J.l_off, P->n_sm, flags, s, P->tuning.terma_ctas_per_sm);
+                      all ? nullptr : S.list_v + J.l_off, P->n_sm, flags, s, P->tuning.terma_ctas_per_sm);
       CH_CUDA(cudaGetLastError());
     }
   } else {

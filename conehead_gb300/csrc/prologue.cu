@@ -854,7 +854,8 @@ __device__ __forceinline__ bool terma_voxel(const float* __restrict__ rho, const
   return true;
 }
 
-// Pass 2, listed voxels: TERMA and its support box for the cone stage.
+// Pass 2, listed voxels (EXACT: all voxels in order where there is no list):
+// TERMA and its support box for the cone stage.
 // Entry e of a beam's list of count voxels; every lane of the warp calls it
 // (the box reduction is warp-wide).
 template <bool EXACT>
@@ -867,7 +868,7 @@ __device__ __forceinline__ void terma_entry(const float* __restrict__ rho, const
     int x = 0, y = 0, z = 0, bad = 0;
     float Tv = 0.0f;
     if (live) {
-      const int v = list_v[e];
+      const int v = EXACT && !list_v ? e : list_v[e];
       z = v % g.n[2];
       const int r = v / g.n[2];
       y = r % g.n[1];
@@ -914,7 +915,7 @@ __device__ __forceinline__ void terma_body(const float* __restrict__ rho, const 
                                            int all_voxels, const int* __restrict__ list_count,
                                            const int* __restrict__ list_v, int* __restrict__ aabb,
                                            int* __restrict__ flags, int cta, int n_ctas) {
-  const int count = *list_count;
+  const int count = list_v ? *list_count : g.n[0] * g.n[1] * g.n[2];
   const int rounds = (count + blockDim.x * n_ctas - 1) / (blockDim.x * n_ctas);
   for (int it = 0; it < rounds; ++it)
     terma_entry<true>(rho, g, b, s, T, inter, all_voxels, count, (it * n_ctas + cta) * blockDim.x + threadIdx.x,
@@ -1275,7 +1276,11 @@ void launch_prologue(const float* rho, const GridDev& g, const BeamDev& b, const
   const int threads = 256;
   const long long lines = (long long)g.n[0] * g.n[1];
   int* list_count = aabb + 6;
-  cull_kernel<<<(unsigned)((lines + 7) / 8), threads, 0, st>>>(g, b, T, inter, all_voxels, list_count, list_v);
+  // without a list (all voxels) the TERMA pass takes them in order and writes
+  // every one: there is nothing to cull or to zero (96^3 with every
+  // intermediate: 20 of 209 us)
+  if (list_v)
+    cull_kernel<<<(unsigned)((lines + 7) / 8), threads, 0, st>>>(g, b, T, inter, all_voxels, list_count, list_v);
   const long long want = (N + threads - 1) / threads;
   const long long cap = (long long)n_sm * ctas_per_sm;
   const int grid = (int)(want < cap ? want : cap);

@@ -5,6 +5,8 @@
   passes: a narrow beam after wide ones equals the narrow beam on a new plan.
 * A ray parallel to the blocking plane is reported by the call that met it.
 * The radiological scatter with an axis above 512 voxels.
+* All intermediates (every voxel in order, no list) against the plain dose, for
+  both cone methods.
 * Map rasters of every row length modulo 4 and of an unaligned buffer.
 """
 import ctypes
@@ -111,6 +113,23 @@ def test_radiological_scatter_of_long_axes(settings, n):
     # water: the same taps and weights, summed in another order
     assert geo.max() > 0
     assert np.abs(rad - geo).max() <= 2e-5 * geo.max()
+
+
+@pytest.mark.parametrize("n", [(2, 3, 5), (1, 1, 33), (31, 9, 29), (40, 28, 47)])
+@pytest.mark.parametrize("method", [0, 1])
+def test_dose_with_all_intermediates(settings, n, method):
+    eng = _engine(settings)
+    eng.set_tuning(cone_method=method)
+    ph = _phantom(n)
+    a = _doses(eng, [_job(eng, ph, settings, 33.0, 12.0, (-3.1, 2.4, -1.9, 2.7))])[0]
+    job = _job(eng, ph, settings, 33.0, 12.0, (-3.1, 2.4, -1.9, 2.7))
+    for _ in range(2):
+        _, inter = eng.run(job, intermediates=True)
+        eng.sync()
+        # the gather adds each voxel's work units in arrival order
+        assert np.abs(job.dose.cpu().numpy() - a).max() <= 1e-5 * a.max()
+    blocked, terma = inter["blocked"].cpu().numpy(), inter["terma"].cpu().numpy()
+    assert terma.max() > 0 and not terma[blocked == 0].any()
 
 
 @pytest.mark.parametrize("cols", [1, 2, 3, 127, 129, 402, 403, 404])
