@@ -266,6 +266,7 @@ struct SpecGrid {
   int plane;               // the plane path (spec_plane_path): A = [Mz][lp] plane-major, no B
   int lp;                  // plane pitch of A on the plane path (nx ny rounded up to 32)
   int skip;                // rows of A without TERMA are not written: their reader goes by the line flags
+  int ahead;               // the y and x passes ask L2 for the lines of a later CTA
   int after;               // the passes start while their predecessors end (launch_after)
 };
 struct SpecLaunch {

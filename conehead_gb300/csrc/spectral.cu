@@ -804,6 +804,12 @@ static void y_pass(const SpecLaunch& L, bool inverse, cudaStream_t st) {
 // gains nothing and its successor's CTAs take its last wave's place.
 constexpr long long SPEC_AFTER_MAX = 6 << 20;
 
+// Lines are asked for ahead where the y and x passes' work array B does not stay in
+// L2 (129 MB): cone stage without / with, one beam at 192^3 (113 MB) 209 / 228 us,
+// at 201^3 (167 MB) 346 / 329, at 256^3 697 / 626; four at 144^3 (191 MB) 282 / 281,
+// 192^3 717 / 675; 16 at 64^3 (67 MB) 98 / 99, 96^3 (226 MB) 324 / 312.
+constexpr long long SPEC_AHEAD_MIN = 18 << 20;   // complex values of B
+
 void launch_spec_beams(SpecLaunch& L, cudaStream_t st) {
   // rows of A without TERMA are neither written nor read where the y pass goes
   // by the line flags (the kernels of lengths to 512): cone stage of 4 beams at 144^3 308 -> 298 us, 7 at 192^3
@@ -811,6 +817,7 @@ void launch_spec_beams(SpecLaunch& L, cudaStream_t st) {
   // SM) costs more than the rows: 32 beams at 128^3 1260 -> 1362.
   L.g.skip = !L.g.plane && std::max(L.g.M[1], L.g.M[2]) <= 512;
   L.g.after = (long long)L.n_beams * L.g.n[0] * L.g.n[1] * L.g.M[2] <= SPEC_AFTER_MAX ? 1 : 0;
+  L.g.ahead = (long long)L.n_beams * L.g.n[0] * L.g.M[1] * L.g.M[2] >= SPEC_AHEAD_MIN ? 1 : 0;
   z_pass(L, false, st);
   if (L.g.plane) {
     // clusters of two along x: consecutive clusters take the same kz plane of

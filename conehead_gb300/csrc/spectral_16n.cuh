@@ -26,4 +26,15 @@ constexpr int r16n_threads() { return 16 * N2 > 256 ? 16 * N2 : 256; }
 template <int N2>
 constexpr int r16n_ctas() { return N2 <= 12 ? 6 : N2 <= 16 ? 5 : N2 <= 20 ? 4 : N2 <= 24 ? 3 : 2; }
 
+// The y and x passes have two or three CTAs per SM, all waiting for memory at
+// their start: each asks L2 for the lines of the CTA SPEC_AHEAD further on, one
+// row of 128 bytes per thread (76 and 228 CTAs ahead: within 1%; 608 in the y
+// pass: nothing gained).  Cone stage without / x alone / both, seven beams at 192^3
+// 1248 / 1205 / 1168 us, 64 mixed beams 2654 / 2608 / 2563.  Nothing gained in the z
+// passes, 1.5% lost in the plane kernel.
+constexpr int SPEC_AHEAD = 152;
+__device__ __forceinline__ void prefetch_row(const float2* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 }  // namespace ch

@@ -27,7 +27,7 @@ constexpr int x_smem() { return (2 * 16 * N2 * 16 + (x_table<N2>() ? 16 * N2 : 0
 template <int N2>
 constexpr int x_ctas() { return N2 <= 10 ? 5 : N2 <= 12 ? 4 : N2 <= 18 ? 3 : 2; }
 
-template <int N2>
+template <int N2, bool AHEAD>
 __global__ void __launch_bounds__(r16n_threads<N2>(), x_ctas<N2>()) spec_x_kernel(SpecLaunch P) {
   constexpr int M = 16 * N2, T = r16n_threads<N2>();
   float2* const xb = spec_sm;                 // exchange, row r at 16 r
@@ -55,6 +55,13 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), x_ctas<N2>()) spec_x_kerne
   static_assert(M <= T, "one table entry per thread");
   const float2 w_mine = x_table<N2>() ? __ldg(P.g.tw[0] + min((int)threadIdx.x, M - 1)) : make_float2(0.0f, 0.0f);
   after_wait();   // S^ and the twiddles are older than any kernel of this call
+  if (AHEAD) {
+    const unsigned next = blockIdx.x + SPEC_AHEAD;
+    if (next < gridDim.x && (int)threadIdx.x < nx) {
+      const int blk2 = next / P.n_beams, ky2 = blk2 / nkb, kz2 = (blk2 - ky2 * nkb) << 4;
+      prefetch_row(P.p[next - blk2 * P.n_beams].b + (size_t)ky2 * L + kz2 + threadIdx.x * xs);
+    }
+  }
   float2 v[16];
   if (threadIdx.x < 16 * N2) {
 #pragma unroll
@@ -161,7 +168,9 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), 1) spec_full_kernel(SpecFu
 
 template <int N2>
 static cudaError_t x_setup() {
-  cudaError_t e = cudaFuncSetAttribute(spec_x_kernel<N2>, cudaFuncAttributeMaxDynamicSharedMemorySize, x_smem<N2>());
+  cudaError_t e = cudaFuncSetAttribute(spec_x_kernel<N2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, x_smem<N2>());
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(spec_x_kernel<N2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, x_smem<N2>());
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(spec_full_kernel<N2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * N2 * 16 * 8);
   return e;
@@ -182,7 +191,8 @@ bool launch_spec_x(const SpecLaunch& L, cudaStream_t st) {
   switch (L.g.M[0]) {
 #define X_CASE(N2)                                                                  \
   case 16 * N2:                                                                     \
-    launch_after(L.g.after, spec_x_kernel<N2>, grid, r16n_threads<N2>(), x_smem<N2>(), st, L); \
+    launch_after(L.g.after, L.g.ahead ? spec_x_kernel<N2, true> : spec_x_kernel<N2, false>, grid, r16n_threads<N2>(), \
+                 x_smem<N2>(), st, L);                                              \
     return true;
     SPEC_N2(X_CASE)
 #undef X_CASE

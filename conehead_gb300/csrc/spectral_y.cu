@@ -23,7 +23,7 @@ extern __shared__ float2 spec_sm[];
 template <int N2>
 constexpr int y_smem() { return (16 * N2 * 16 + 16 * N2) * 8; }
 
-template <bool INV, int N2>
+template <bool INV, int N2, bool AHEAD>
 __global__ void __launch_bounds__(r16n_threads<N2>(), r16n_ctas<N2>()) spec_y_kernel(SpecLaunch P) {
   constexpr int M = 16 * N2, T = r16n_threads<N2>();
   float2* const xb = spec_sm;                 // exchange, row r at 16 r
@@ -39,7 +39,13 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), r16n_ctas<N2>()) spec_y_ke
   after_trigger();
   const float2 w_mine = __ldg(P.g.tw[1] + min((int)threadIdx.x, M - 1));
   after_wait();
-  const unsigned char* const lines = P.g.skip && bm.l ? bm.l + x * ny : nullptr;
+  const unsigned char* const lines = !INV && P.g.skip && bm.l ? bm.l + x * ny : nullptr;
+  if (AHEAD) {
+    const unsigned next = blockIdx.x + SPEC_AHEAD;
+    const int x2 = next / nkb, kz2 = (next - x2 * nkb) << 4, row = threadIdx.x;
+    if (next < gridDim.x && row < (INV ? M : ny) && (!lines || bm.l[x2 * ny + row] != 0))
+      prefetch_row((INV ? bm.b + ((size_t)x2 * M + row) * L : bm.a + ((size_t)x2 * ny + row) * L) + kz2);
+  }
   // the inputs are in flight while the table is published
   float2 v[16], a[N2];
   if (!INV) {
@@ -107,9 +113,11 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), r16n_ctas<N2>()) spec_y_ke
 
 template <int N2>
 static cudaError_t y_setup() {
-  cudaError_t e = cudaFuncSetAttribute(spec_y_kernel<false, N2>, cudaFuncAttributeMaxDynamicSharedMemorySize, y_smem<N2>());
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(spec_y_kernel<true, N2>, cudaFuncAttributeMaxDynamicSharedMemorySize, y_smem<N2>());
+  cudaError_t e = cudaSuccess;
+  void (*const k[4])(SpecLaunch) = {spec_y_kernel<false, N2, false>, spec_y_kernel<false, N2, true>,
+                                    spec_y_kernel<true, N2, false>, spec_y_kernel<true, N2, true>};
+  for (auto f : k)
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, y_smem<N2>());
   return e;
 }
 
@@ -126,12 +134,12 @@ cudaError_t setup_spec_y() {
 bool launch_spec_y(const SpecLaunch& L, bool inverse, cudaStream_t st) {
   const dim3 grid(L.g.n[0] * (L.g.M[2] / 16), L.n_beams);
   switch (L.g.M[1]) {
-#define Y_CASE(N2)                                                                     \
-  case 16 * N2:                                                                        \
-    if (inverse)                                                                       \
-      launch_after(L.g.after, spec_y_kernel<true, N2>, grid, r16n_threads<N2>(), y_smem<N2>(), st, L); \
-    else                                                                               \
-      launch_after(L.g.after, spec_y_kernel<false, N2>, grid, r16n_threads<N2>(), y_smem<N2>(), st, L); \
+#define Y_CASE(N2)                                                                                     \
+  case 16 * N2:                                                                                        \
+    launch_after(L.g.after,                                                                            \
+                 inverse ? (L.g.ahead ? spec_y_kernel<true, N2, true> : spec_y_kernel<true, N2, false>) \
+                         : (L.g.ahead ? spec_y_kernel<false, N2, true> : spec_y_kernel<false, N2, false>), \
+                 grid, r16n_threads<N2>(), y_smem<N2>(), st, L);                                       \
     return true;
     SPEC_N2(Y_CASE)
 #undef Y_CASE

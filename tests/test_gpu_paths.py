@@ -3,6 +3,7 @@
 * One-launch prologue (few small beams) against the list of a larger batch.
 * Rows without TERMA, which are neither written nor read between the z and y
   passes: a narrow beam after wide ones equals the narrow beam on a new plan.
+* Passes that ask L2 for lines ahead (large batches) against one beam at a time.
 * A ray parallel to the blocking plane is reported by the call that met it.
 * The radiological scatter with an axis above 512 voxels.
 * All intermediates (every voxel in order, no list) against the plain dose, for
@@ -82,6 +83,20 @@ def test_rows_without_terma(settings, n, beams):
     for a, b in zip(_doses(used, jobs(used, narrow)), _doses(new, jobs(new, narrow))):
         assert b.max() > 0
         assert np.array_equal(a, b)
+
+
+# the batch's work array is past 18 << 20 values, one beam's is not
+@pytest.mark.parametrize("n,beams", [((150, 131, 155), 3), ((70, 250, 129), 4), ((33, 40, 200), 32)])
+def test_lines_asked_for_ahead(settings, n, beams):
+    eng = _engine(settings)
+    ph = _phantom(n, (0.2, 0.2, 0.2))
+    field = (-3.1, 2.4, -1.9, 2.7)
+    jobs = [_job(eng, ph, settings, 23.0 * k % 360.0, 5.0 * k, field) for k in range(beams)]
+    together = _doses(eng, jobs)
+    for job, a in zip(jobs, together):
+        b = _doses(eng, [job])[0]
+        assert b.max() > 0
+        assert np.abs(a - b).max() <= TOL * b.max()
 
 
 def test_parallel_ray_is_reported_once(settings):
