@@ -693,6 +693,21 @@ BeamDev make_beam(const ch_beam& in, const ch_grid& g, int samples) {
   b.vyw = (b.vy[0] * w0 + b.vy[1] * w1) + b.vy[2] * w2;
   b.vywf = (b.vyf[0] * b.srcf[0] + b.vyf[1] * b.srcf[1]) + b.vyf[2] * b.srcf[2];
   b.geom_f32 = in.geom_f32;
+  b.pairs = in.geom_f32 ? 0 : 1;
+  auto low = [&](double v, double lo, double hi) {   // its low part; |v| is 0 or in [lo, hi]
+    const double a = std::fabs(v);
+    if (!(a == 0.0 || (a >= lo && a <= hi))) b.pairs = 0;
+    return (float)(v - (double)(float)v);
+  };
+  for (int k = 0; k < 3; ++k) {
+    b.srcl[k] = low(in.src[k], 1e-12, 1e6);
+    b.vyl[k] = low(b.vy[k], 1e-18, 1e3);
+    b.m0l[k] = low(b.m0[k], 1e-18, 1e3);
+    b.m2l[k] = low(b.m2[k], 1e-18, 1e3);
+    if (!(std::fabs((double)g.origin[k]) <= 1e6 && (double)g.n[k] * g.spacing[k] <= 1e6)) b.pairs = 0;
+  }
+  b.vywh = (float)b.vyw;
+  b.vywl = low(b.vyw, 1e-12, 1e9);
   const double nS = b.vy[0] * b.src[0] + b.vy[1] * b.src[1] + b.vy[2] * b.src[2];
   const double m0S = b.m0[0] * b.src[0] + b.m0[1] * b.src[1] + b.m0[2] * b.src[2];
   const double m2S = b.m2[0] * b.src[0] + b.m2[1] * b.src[1] + b.m2[2] * b.src[2];

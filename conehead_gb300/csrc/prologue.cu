@@ -98,6 +98,50 @@ __device__ __forceinline__ void ray_to_source(const BeamDev& b, const float* p, 
   }
 }
 
+// The float64 projection in pairs of float32 (48 bits): products with their
+// exact residual, Knuth's two-sums, a quotient with one correction.  px and pz
+// differ from project_exact_mixed's where that value lies within about 2^-46 of
+// the terms of a float32 tie.  A float64 instruction holds the pipe of an SM quarter
+// for 64 cycles, and the 33 of this projection were two thirds of what it did.
+// Prologue, float64 / pairs: one beam at 64^3 29 / 24 us, 150 x 130 x 92 126 / 118, 32
+// beams 5 x 5 cm at 128^3 441 / 423, 64 mixed beams 2686 / 2525, nine MLC beams 1048 /
+// 988, seven at 192^3 (long walks) 457 / 459.  Intermediates keep the float64 bits.
+struct Pair {
+  float h, l;
+};
+__device__ __forceinline__ Pair two_sum(float a, float b) {
+  const float s = fadd(a, b), bb = fsub(s, a);
+  return {s, fadd(fsub(a, fsub(s, bb)), fsub(b, bb))};
+}
+__device__ __forceinline__ Pair pair_dot(const float* vh, const float* vl, const float* r) {
+  Pair p[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    p[k].h = fmul(vh[k], r[k]);
+    p[k].l = __fmaf_rn(vl[k], r[k], __fmaf_rn(vh[k], r[k], -p[k].h));
+  }
+  const Pair a = two_sum(p[0].h, p[1].h), t = two_sum(a.h, p[2].h);
+  return {t.h, fadd(fadd(fadd(p[0].l, p[1].l), a.l), fadd(p[2].l, t.l))};
+}
+__device__ __forceinline__ bool project_pairs(const BeamDev& b, const float* rd, float& px, float& pz) {
+  const Pair d = pair_dot(b.vyf, b.vyl, rd);
+  const float h = fadd(d.h, d.l), l = fadd(fsub(d.h, h), d.l);
+  if (!(fabsf(h) > 2e-6f)) return false;   // parallel, or nearly
+  const float q1 = __fdividef(-b.vywh, h);
+  const float q2 = __fdividef(fsub(__fmaf_rn(-q1, l, __fmaf_rn(-q1, h, -b.vywh)), b.vywl), h);
+  float pp[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float m = fmul(q1, rd[k]), e = __fmaf_rn(q2, rd[k], __fmaf_rn(q1, rd[k], -m));
+    const Pair s = two_sum(b.srcf[k], m);
+    pp[k] = fadd(s.h, fadd(s.l, e));
+  }
+  const Pair x = pair_dot(b.m0f, b.m0l, pp), z = pair_dot(b.m2f, b.m2l, pp);
+  px = fadd(x.h, x.l);
+  pz = fadd(z.h, z.l);
+  return true;
+}
+
 __device__ __forceinline__ bool project_exact(const BeamDev& b, const float* rd, float& px, float& pz) {
   return b.geom_f32 ? project_exact_f32(b, rd, px, pz) : project_exact_mixed(b, rd, px, pz);
 }
@@ -425,9 +469,9 @@ __device__ __forceinline__ double div_count(float v, double n, double inv_n) {
 // took 32 rounds), and a map's voxels went through those rounds and then again
 // through a per-lane loop with a float64 division per change of value; then by
 // float64 issue (sums, exact samples).  Prologues, start of that work / now:
-// nine MLC beams on 140 x 101 x 112 8.59 / 1.22 ms, 64 mixed jaw beams 5.18 /
-// 2.69 ms, 32 beams 5 x 5 cm on 128^3 0.88 / 0.45 ms (the walk and the cull
-// below have their share; this function alone, last step: 1.69 -> 1.22, 2.94 ->
+// nine MLC beams on 140 x 101 x 112 8.59 / 0.99 ms, 64 mixed jaw beams 5.18 /
+// 2.53 ms, 32 beams 5 x 5 cm on 128^3 0.88 / 0.42 ms (the walk, the projection and
+// the cull have their share; this function alone, last step: 1.69 -> 1.22, 2.94 ->
 // 2.69, 0.490 -> 0.446 ms).
 //
 // EXACT: the bits of the reference's float64 sum also for maps (where the
@@ -812,7 +856,8 @@ __device__ __forceinline__ bool terma_voxel(const float* __restrict__ rho, const
   const float deff = radiological_depth(rho, g, x, y, z, rd);
   // ---- off-axis distance (exact mirror)
   float px = 0.0f, pz = 0.0f;
-  if (!project_exact(b, rd, px, pz)) bad = 1;
+  if (EXACT || !b.pairs || !project_pairs(b, rd, px, pz))
+    if (!project_exact(b, rd, px, pz)) bad = 1;
   const float oad = __fsqrt_rn(fadd(fmul(px, px), fmul(pz, pz)));
   // ---- fluence (float32 evaluation of the reference's float64 formula)
   const float mag = __fsqrt_rn(fadd(fadd(fmul(rd[0], rd[0]), fmul(rd[1], rd[1])), fmul(rd[2], rd[2])));
