@@ -1270,11 +1270,12 @@ ch_status enqueue_spectral(ch_plan* P, const BatchPlan& B, const Scratch& S, boo
 // FUSED_MAX_LINES (x, y) lines in all and, by the opening times the grid's
 // length along the beam, FUSED_MAX_CHUNKS chunks of 32 voxels in the field.
 // Measured, whole calls with a turned collimator, two launches and a copy
-// against one: 64^3 12 x 12 cm 98.7 / 89.8 us, 4 beams 5 x 5 cm on 64^3
-// (16384 lines) 121 / 117, 96^3 8 x 8 cm (9216) 109.5 / 111.2, 128^3 5 x 5 cm
-// (16384) 134.7 / 133.4, 7 x 7 cm 146 / 160, 150 x 130 lines 217 / 230: a warp
-// per line costs more than the cull once lines outnumber the resident warps.
-constexpr int FUSED_MAX_LINES = 8192, FUSED_MAX_CHUNKS = 6000;
+// against one: 24^3 5 x 5 cm 65 / 57 us, 64^3 5 x 5 cm 78 / 67, 64^3 12 x 12 cm 87 / 83,
+// 64^3 whole (8192 chunks) 89 / 79, 90 x 90 x 32 whole (8100) 103 / 90, 24 x 24 x 480
+// 80 / 76, two beams on 64^3 (8192 lines) 87 / 85, 96^3 8 x 8 cm (9216) 102 / 104, four
+// beams on 64^3 (16384) 107 / 111, two on 96^3 119 / 131: a warp per line costs more
+// than the list once lines outnumber the resident warps.
+constexpr int FUSED_MAX_LINES = 8192, FUSED_MAX_CHUNKS = 9000;
 bool fused_prologue(const BatchPlan& B) {
   if (B.jobs.size() > FUSED_MAX_BEAMS) return false;
   double vox = 0.0;

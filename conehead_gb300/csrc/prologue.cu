@@ -469,8 +469,8 @@ __device__ __forceinline__ double div_count(float v, double n, double inv_n) {
 // took 32 rounds), and a map's voxels went through those rounds and then again
 // through a per-lane loop with a float64 division per change of value; then by
 // float64 issue (sums, exact samples).  Prologues, start of that work / now:
-// nine MLC beams on 140 x 101 x 112 8.59 / 0.99 ms, 64 mixed jaw beams 5.18 /
-// 2.53 ms, 32 beams 5 x 5 cm on 128^3 0.88 / 0.42 ms (the walk, the projection and
+// nine MLC beams on 140 x 101 x 112 8.59 / 0.91 ms, 64 mixed jaw beams 5.18 /
+// 2.05 ms, 32 beams 5 x 5 cm on 128^3 0.88 / 0.33 ms (the walk, the projection and
 // the cull have their share; this function alone, last step: 1.69 -> 1.22, 2.94 ->
 // 2.69, 0.490 -> 0.446 ms).
 //
@@ -746,92 +746,107 @@ __device__ __forceinline__ void load_record(const PrologueBeam* __restrict__ rec
   __syncthreads();
 }
 
-// Every beam of a batch in one launch (blockIdx.y = beam), lpc lines per CTA (a
-// multiple of 16, at most 128).  Lane pairs test a line each (line_outside), so
-// a warp rejects 16 lines in the instructions of one; the lines that pass are
-// gathered in shared memory and taken by the warps one at a time: candidates of
-// up to 1024 voxels as one ballot per 32, kept by lane, then one add to the
-// beam's list count for all of them.  A warp per line spent 32 lanes on every
-// line test (80% of the lines fail it) and one add, whose result it waited for,
-// on every 32 voxels: 32 beams at 128^3 157 -> 75 us, 64 mixed beams 660 -> 305
-// us (an empty CTA now returns before it copies its record).
-__global__ void __launch_bounds__(256) cull_batch_kernel(const PrologueBeam* __restrict__ recs, int lpc) {
+// Voxels [x, y) of a line that the beam may reach: line_outside's argument,
+// solved for z.  With depth, x0 and x2 linear along the line, "xb >= cx_lo - M"
+// times depth, M the line's largest margin, is linear too: its end values say
+// whether it holds everywhere, nowhere or up to a crossing.  A line that comes
+// near the source plane is kept whole.  A NaN restricts nothing.
+__device__ __forceinline__ int2 line_span(const GridDev& g, const BeamDev& b, float px, float py) {
+  const int nz = g.n[2];
+  if (!b.cull_enable) return make_int2(0, nz);
+  const float kk = fabsf(b.a_K);
+  const float n_xy = b.vyf[0] * px + b.vyf[1] * py, x0_xy = b.a_m0S - (b.m0f[0] * px + b.m0f[1] * py);
+  const float x2_xy = b.a_m2S - (b.m2f[0] * px + b.m2f[1] * py);
+  float depth[2], x0[2], x2[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const float pz = voxel_centre(g.origin[2], g.spacing[2], e ? nz - 1 : 0);
+    depth[e] = (n_xy + b.vyf[2] * pz) - b.a_nS;
+    x0[e] = x0_xy - b.m0f[2] * pz;
+    x2[e] = x2_xy - b.m2f[2] * pz;
+  }
+  if (!(depth[0] > 0.2f * kk && depth[1] > 0.2f * kk)) return make_int2(0, nz);
+  const float i0 = 1.0f / depth[0], i1 = 1.0f / depth[1];
+  const float lat = fmaxf(fmaxf(fabsf(x0[0]), fabsf(x2[0])) * i0, fmaxf(fabsf(x0[1]), fabsf(x2[1])) * i1);
+  const float M = b.cull_margin_k * kk * fmaxf(i0, i1) * (1.0f + lat) + 0.02f;
+  float lo = 0.0f, hi = (float)(nz - 1);
+  bool none = false;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float* v = k < 2 ? x0 : x2;
+    const float c = k < 2 ? b.a_c0 : b.a_c2;
+    const float edge = k == 0 ? b.cx_lo : k == 1 ? b.cx_hi : k == 2 ? b.cz_lo : b.cz_hi;
+    const float w = (k & 1) ? (edge - c) + M : (c - edge) + M, K = (k & 1) ? b.a_K : -b.a_K;
+    const float g0 = w * depth[0] + K * v[0], g1 = w * depth[1] + K * v[1];
+    none = none || (g0 < 0.0f && g1 < 0.0f);
+    const float t = g0 / (g0 - g1) * (float)(nz - 1);
+    if (g0 < 0.0f && g1 >= 0.0f) lo = fmaxf(lo, t - 0.01f);
+    if (g1 < 0.0f && g0 >= 0.0f) hi = fminf(hi, t + 0.01f);
+  }
+  const int z0 = max((int)ceilf(lo), 0), z1 = min((int)floorf(hi), nz - 1) + 1;
+  return none || z1 <= z0 ? make_int2(0, 0) : make_int2(z0, z1);
+}
+
+// Every beam of a batch in one launch (blockIdx.y = beam), lpw lines per warp (at
+// most 32), one per lane: its span of voxels, one add to the beam's list count
+// for the whole warp, then line by line the list entries and, where only these
+// lines are read, TERMA's zeros in 16-byte stores.
+//
+// Issue bound at first: a warp per line, a projection per voxel and an add, whose
+// result it waited for, per 32 voxels / lane pairs testing lines and the
+// projections on those that passed (230 instructions per 32 voxels, 83% issue
+// active) / this, which writes 8 bytes per listed voxel: 32 beams at 128^3 157 / 75 /
+// 30 us, seven at 192^3 130 / 100 / 19, 64 mixed beams 671 / 305 / 63.  The TERMA launch
+// gained too, its chunks running along lines in order (64 mixed beams 2.22 -> 1.98
+// ms).  Prologues, last step: 424 -> 332 us, 457 -> 328, 2523 -> 2050.
+__global__ void __launch_bounds__(256) cull_batch_kernel(const PrologueBeam* __restrict__ recs, int lpw) {
   __shared__ PrologueBeam R;
-  __shared__ short kept[128];
-  __shared__ int n_kept;
   const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31, l0 = blockIdx.x * lpc;
+  const int lane = threadIdx.x & 31;
   after_trigger();
   after_wait();
   {
     const PrologueBeam& G = recs[blockIdx.y];
-    if (l0 >= G.g.n[0] * G.g.n[1]) return;   // whole CTA
+    if ((int)(blockIdx.x * (blockDim.x >> 5)) * lpw >= G.g.n[0] * G.g.n[1]) return;   // whole CTA
   }
-  if (threadIdx.x == 0) n_kept = 0;
   load_record(recs, R);
   const GridDev& g = R.g;
-  const BeamDev& b = R.b;
-  const int n1 = g.n[1], nz = g.n[2], lines = g.n[0] * n1;
-  if ((threadIdx.x >> 1) < lpc) {             // whole warps
-    const int i = threadIdx.x >> 1, line = min(l0 + i, lines - 1);
-    const int x = line / n1, y = line - x * n1;
-    const bool out = b.cull_enable && line_outside(g, b, voxel_centre(g.origin[0], g.spacing[0], x),
-                                                   voxel_centre(g.origin[1], g.spacing[1], y));
-    const bool mine = (lane & 1) == 0 && l0 + i < lines;
-    const unsigned m = __ballot_sync(full, mine && !out);
-    int base = 0;
-    if (lane == 0 && m) base = atomicAdd(&n_kept, __popc(m));
-    base = __shfl_sync(full, base, 0);
-    if (mine && !out) kept[base + __popc(m & ((1u << lane) - 1u))] = (short)i;
-    if (mine && out) {
-      R.line_any[line] = 0;
-    }
+  const int n1 = g.n[1], nz = g.n[2], lines = g.n[0] * n1, quads = g.zp >> 2;
+  const int line0 = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * lpw;
+  const int mine = min(lpw, lines - line0);    // this warp's lines
+  if (mine <= 0) return;                       // whole warp
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  int2 span = make_int2(0, 0);
+  if (lane < mine) {
+    const int line = line0 + lane, x = line / n1, y = line - x * n1;
+    span = line_span(g, R.b, voxel_centre(g.origin[0], g.spacing[0], x), voxel_centre(g.origin[1], g.spacing[1], y));
+    R.line_any[line] = span.y > span.x ? 1 : 0;
   }
-  __syncthreads();
   if (R.zero_all) {                            // the gather reads TERMA anywhere
-    const int n = min(lpc, lines - l0) * g.zp;
-    float* T = R.T + (size_t)l0 * g.zp;
-    for (int e = threadIdx.x; e < n; e += blockDim.x) T[e] = 0.0f;
+    float4* T4 = reinterpret_cast<float4*>(R.T + (size_t)line0 * g.zp);
+    for (int e = lane; e < mine * quads; e += 32) T4[e] = zero;
   }
-  for (int k = threadIdx.x >> 5; k < n_kept; k += blockDim.x >> 5) {
-    const int line = l0 + kept[k];
-    const int x = line / n1, y = line - x * n1;
-    float pos[3] = {voxel_centre(g.origin[0], g.spacing[0], x), voxel_centre(g.origin[1], g.spacing[1], y), 0.0f};
-    bool any = false;
-    for (int zb = 0; zb < nz; zb += 1024) {
-      const int chunks = (min(nz - zb, 1024) + 31) >> 5;
-      unsigned mine = 0;                       // candidates of chunk `lane`
-      for (int c = 0; c < chunks; ++c) {
-        const int z = zb + 32 * c + lane;
-        pos[2] = voxel_centre(g.origin[2], g.spacing[2], z);
-        const unsigned m = __ballot_sync(full, z < nz && cull_candidate(b, pos));
-        if (lane == c) mine = m;
-      }
-      int incl = __popc(mine);
+  const int count = span.y - span.x;
+  int incl = count;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int up = __shfl_up_sync(full, incl, o);
-        if (lane >= o) incl += up;
-      }
-      const int total = __shfl_sync(full, incl, 31);
-      if (total == 0) continue;
-      any = true;
-      int base = 0;
-      if (lane == 0) base = atomicAdd(R.aabb + 6, total);
-      base = __shfl_sync(full, base, 0);
-      const int before = incl - __popc(mine);
-      for (int c = 0; c < chunks; ++c) {
-        const unsigned m = __shfl_sync(full, mine, c);
-        const int at = base + __shfl_sync(full, before, c);
-        if ((m >> lane) & 1u)
-          R.list_v[at + __popc(m & ((1u << lane) - 1u))] = line * nz + zb + 32 * c + lane;
-      }
+  for (int o = 1; o < 32; o <<= 1) {
+    const int up = __shfl_up_sync(full, incl, o);
+    if (lane >= o) incl += up;
+  }
+  const int total = __shfl_sync(full, incl, 31);
+  if (total == 0) return;
+  int base = 0;
+  if (lane == 0) base = atomicAdd(R.aabb + 6, total);
+  base = __shfl_sync(full, base, 0) + incl - count;
+  for (unsigned m = __ballot_sync(full, count > 0); m; m &= m - 1) {
+    const int l = __ffs(m) - 1, line = line0 + l;
+    const int n = __shfl_sync(full, count, l), v = line * nz + __shfl_sync(full, span.x, l);
+    int* dst = R.list_v + __shfl_sync(full, base, l);
+    for (int i = lane; i < n; i += 32) dst[i] = v + i;
+    if (!R.zero_all) {
+      float4* T4 = reinterpret_cast<float4*>(R.T + (size_t)line * g.zp);
+      for (int e = lane; e < quads; e += 32) T4[e] = zero;
     }
-    if (!R.zero_all && any) {
-      float* Tl = R.T + (size_t)line * g.zp;
-      for (int z = lane; z < nz; z += 32) Tl[z] = 0.0f;
-    }
-    if (lane == 0) R.line_any[line] = any ? 1 : 0;
   }
 }
 
@@ -1023,8 +1038,7 @@ __global__ void __launch_bounds__(256, 3) terma_batch_kernel(const PrologueBeam*
 }
 
 // Cull and TERMA of a few small beams in one launch, a warp per (x, y) line:
-// the line test, the span of its candidate voxels, then TERMA of the span 32
-// voxels at a time and zeros beside it (on lines without candidates nothing:
+// the span of its candidate voxels, then TERMA of the span 32 voxels at a time and zeros beside it (on lines without candidates nothing:
 // line_any says so).  No list, no counters to reset, and the records come as a
 // kernel parameter: where the beams' voxels do not fill the SMs for long, the
 // time is that of launches and of one chunk's latency, and this needs one
@@ -1041,26 +1055,17 @@ __global__ void __launch_bounds__(256, 3) prologue_fused_kernel(const __grid_con
   if (line >= g.n[0] * g.n[1]) return;   // whole warp
   const int x = line / g.n[1], y = line - x * g.n[1], nz = g.n[2];
   float pos[3] = {voxel_centre(g.origin[0], g.spacing[0], x), voxel_centre(g.origin[1], g.spacing[1], y), 0.0f};
-  int lo = nz, hi = -1;
-  if (!(b.cull_enable && line_outside(g, b, pos[0], pos[1])))
-    for (int z0 = 0; z0 < nz; z0 += 32) {
-      pos[2] = voxel_centre(g.origin[2], g.spacing[2], z0 + lane);
-      const unsigned m = __ballot_sync(0xffffffffu, z0 + lane < nz && cull_candidate(b, pos));
-      if (m) {
-        lo = min(lo, z0 + __ffs(m) - 1);
-        hi = z0 + 31 - __clz(m);
-      }
-    }
-  if (lane == 0) R.line_any[line] = hi >= 0;
-  if (hi < 0) return;
+  const int2 span = line_span(g, b, pos[0], pos[1]);
+  const int lo = span.x, hi = span.y - 1;
+  if (lane == 0) R.line_any[line] = hi >= lo;
+  if (hi < lo) return;
   float* const T = R.T + (size_t)line * g.zp;
   for (int z = lane; z < lo; z += 32) T[z] = 0.0f;
   int bad = 0;
   for (int z = lo + lane; z - lane <= hi; z += 32) {
     float Tv = 0.0f;
     pos[2] = voxel_centre(g.origin[2], g.spacing[2], z);
-    if (z <= hi && cull_candidate(b, pos))
-      terma_voxel<false>(R.rho, g, b, R.s, Inter{}, 0, x, y, z, 0, pos, bad, Tv);
+    if (z <= hi) terma_voxel<false>(R.rho, g, b, R.s, Inter{}, 0, x, y, z, 0, pos, bad, Tv);
     if (z < nz) T[z] = Tv;
     __syncwarp();
   }
@@ -1339,10 +1344,11 @@ void launch_prologue(const float* rho, const GridDev& g, const BeamDev& b, const
 void launch_prologue_batch(const PrologueBeam* recs, int n_beams, long long max_voxels, long long max_lines,
                            int n_sm, int* flags, int* work, cudaStream_t st, int ctas_per_sm) {
   const int threads = 256;
-  // lines per CTA: enough CTAs for every SM's resident ones, at most 128 lines
-  const long long per = max_lines * n_beams / ((long long)n_sm * 8);
-  const int lpc = (int)std::min(128ll, std::max(16ll, per / 16 * 16));
-  launch_after(true, cull_batch_kernel, dim3((unsigned)((max_lines + lpc - 1) / lpc), n_beams), threads, 0, st, recs, lpc);
+  // lines per warp: enough warps for every SM's resident ones, at most 32 lines
+  int lpw = 4;
+  while (lpw < 32 && max_lines * n_beams > (long long)n_sm * 64 * lpw) lpw *= 2;
+  const long long per = lpw * (threads / 32);
+  launch_after(true, cull_batch_kernel, dim3((unsigned)((max_lines + per - 1) / per), n_beams), threads, 0, st, recs, lpw);
   // persistent: at most the resident CTAs (3 per SM at 80 registers), fewer
   // for small batches; the warps share all beams' chunks
   const long long want = ((long long)n_beams * max_voxels + threads - 1) / threads;

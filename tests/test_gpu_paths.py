@@ -54,7 +54,7 @@ def _doses(eng, jobs):
     return [j.dose.cpu().numpy() for j in jobs]
 
 
-# 8 x 1024 lines is the most of the one-launch prologue; 91 x 91 is past it
+# 8192 lines are the most of the one-launch prologue; 91 x 91 is past it
 @pytest.mark.parametrize("n", [(5, 6, 7), (1, 1, 40), (40, 1, 33), (33, 28, 47), (64, 128, 32), (91, 91, 20)])
 @pytest.mark.parametrize("beams", [1, 4])
 def test_one_launch_prologue_equals_the_list(settings, n, beams):
