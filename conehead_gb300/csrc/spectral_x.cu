@@ -130,41 +130,51 @@ __global__ void __launch_bounds__(r16n_threads<N2>(), x_ctas<N2>()) spec_x_kerne
 
 // Forward transform of full lines in place (S^): element i of line (o, c),
 // c < 16, at o1 os1 + o2 os2 + c cs + i is with o = o1 nb + o2; the z axis
-// multiplies by the twist first (spectral_z.cu).
+// multiplies by the twist first (spectral_z.cu).  Lanes run along whichever of
+// line and element is contiguous, with the exchange of the y or of the z passes
+// (lanes across the lines of the z axis read 8 bytes of every 32: 201^3 364 -> 138 us).
 template <int N2>
 __global__ void __launch_bounds__(r16n_threads<N2>(), 1) spec_full_kernel(SpecFull F) {
-  constexpr int M = 16 * N2;
   float2* const xb = spec_sm;
-  const int c = threadIdx.x & 15, h = threadIdx.x >> 4;
+  const int t = threadIdx.x;
+  const bool along = F.is == 1;
   const int o1 = blockIdx.x / F.nb, o2 = blockIdx.x - o1 * F.nb;
-  float2* const line = F.data + (size_t)o1 * F.os1 + (size_t)o2 * F.os2 + (size_t)c * F.cs;
-  if (threadIdx.x < 16 * N2) {
+  float2* const data = F.data + (size_t)o1 * F.os1 + (size_t)o2 * F.os2;
+  // slot of row (n2, k1) of line c
+  const int sc = along ? 17 * N2 : 1, sn = along ? 17 : 16, sk = along ? 1 : 16 * N2;
+  if (t < 16 * N2) {
+    const int n2 = along ? t % N2 : t >> 4, c = along ? t / N2 : t & 15;
+    const float2* const line = data + (size_t)c * F.cs;
     float2 v[16];
 #pragma unroll
     for (int n1 = 0; n1 < 16; ++n1) {
-      const int i = N2 * n1 + h;
+      const int i = N2 * n1 + n2;
       v[n1] = line[(size_t)i * F.is];
       if (F.tq) v[n1] = cmul(v[n1], __ldg(F.tq + i));
     }
     dft16<false>(v);
 #pragma unroll
     for (int m = 0; m < 16; ++m) {
-      float2 t = v[4 * (m & 3) + (m >> 2)];
-      if (m > 0) t = cmul(t, __ldg(F.tw + h * m));
-      xb[(m * N2 + h) * 16 + c] = t;
+      float2 y = v[4 * (m & 3) + (m >> 2)];
+      if (m > 0) y = cmul(y, __ldg(F.tw + n2 * m));
+      xb[m * sk + n2 * sn + c * sc] = y;
     }
   }
   __syncthreads();
-  if (threadIdx.x < 256) {
+  if (t < 256) {
+    const int k1 = along ? t & 15 : t >> 4, c = along ? t >> 4 : t & 15;
+    float2* const line = data + (size_t)c * F.cs;
     float2 a[N2];
 #pragma unroll
-    for (int n2 = 0; n2 < N2; ++n2) a[n2] = xb[(h * N2 + n2) * 16 + c];
+    for (int n2 = 0; n2 < N2; ++n2) a[n2] = xb[k1 * sk + n2 * sn + c * sc];
     Dft<false, N2>::run(a);
 #pragma unroll
-    for (int k2 = 0; k2 < N2; ++k2) line[(size_t)(h + 16 * k2) * F.is] = a[k2];
+    for (int k2 = 0; k2 < N2; ++k2) line[(size_t)(k1 + 16 * k2) * F.is] = a[k2];
   }
-  (void)M;
 }
+
+template <int N2>
+constexpr int full_smem() { return 16 * 17 * N2 * 8; }
 
 template <int N2>
 static cudaError_t x_setup() {
@@ -172,7 +182,7 @@ static cudaError_t x_setup() {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(spec_x_kernel<N2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, x_smem<N2>());
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(spec_full_kernel<N2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * N2 * 16 * 8);
+    e = cudaFuncSetAttribute(spec_full_kernel<N2>, cudaFuncAttributeMaxDynamicSharedMemorySize, full_smem<N2>());
   return e;
 }
 
@@ -204,7 +214,7 @@ bool launch_spec_full(const SpecFull& F, int M, unsigned blocks, cudaStream_t st
   switch (M) {
 #define F_CASE(N2)                                                                  \
   case 16 * N2:                                                                     \
-    spec_full_kernel<N2><<<blocks, r16n_threads<N2>(), 16 * N2 * 16 * 8, st>>>(F);  \
+    spec_full_kernel<N2><<<blocks, r16n_threads<N2>(), full_smem<N2>(), st>>>(F);  \
     return true;
     SPEC_N2(F_CASE)
 #undef F_CASE
