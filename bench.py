@@ -846,8 +846,8 @@ def run_ours(args):
             "config": config(args),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                          "frac": achieved / hbm_peak, "traffic": traffic,
-                         "kernel": (("spectral cone stage, plane path (spec_z_forward_plane, spec_plane, "
-                                     "spec_z_inverse_plane)" if plane_path(ph.size) else
+                         "kernel": (("spectral cone stage, plane path (spec_z_forward_kernel, spec_plane_kernel, "
+                                     "spec_z_inverse_kernel)" if plane_path(ph.size) else
                                      "spectral cone stage (spec_z_forward, spec_y, spec_x, spec_y, spec_z_inverse)")
                                     if method == "spectral" else "cone_gather_kernel"),
                          "algorithmic_bytes_per_step": alg_bytes,

@@ -296,8 +296,9 @@ ch_status ch_cone_directions(ch_plan* plan, float* out_dev, void* stream);
  * cone_method: how the collapsed-cone stage (conehead/conehead.py:385-488)
  *   is evaluated.  CH_CONE_SPECTRAL (default): the stage is one linear
  *   convolution with the tap stencil of all cone walks, applied through
- *   forward and inverse 3-D FFTs of period >= 2n - 1 per axis (grids whose
- *   periods exceed the limit fall back to the gather).  CH_CONE_GATHER: the
+ *   forward and inverse 3-D FFTs of lengths >= 2n - 1 along x and y and >= n
+ *   along z (grids beyond 4096 points per axis or 2^28 in all fall back to the
+ *   gather).  CH_CONE_GATHER: the
  *   tap stencil is walked tile by tile (shared-memory windows, no atomics but
  *   one add per output and work unit).  Both give the reference's dose.
  * dir_group: unique directions per gather work unit, 1..1024 (default 16);
