@@ -469,8 +469,8 @@ __device__ __forceinline__ double div_count(float v, double n, double inv_n) {
 // took 32 rounds), and a map's voxels went through those rounds and then again
 // through a per-lane loop with a float64 division per change of value; then by
 // float64 issue (sums, exact samples).  Prologues, start of that work / now:
-// nine MLC beams on 140 x 101 x 112 8.59 / 0.91 ms, 64 mixed jaw beams 5.18 /
-// 2.05 ms, 32 beams 5 x 5 cm on 128^3 0.88 / 0.33 ms (the walk, the projection and
+// nine MLC beams on 140 x 101 x 112 8.59 / 0.87 ms, 64 mixed jaw beams 5.18 /
+// 1.86 ms, 32 beams 5 x 5 cm on 128^3 0.88 / 0.31 ms (the walk, the projection and
 // the cull have their share; this function alone, last step: 1.69 -> 1.22, 2.94 ->
 // 2.69, 0.490 -> 0.446 ms).
 //
@@ -563,6 +563,11 @@ __device__ __forceinline__ double blocked_fraction(const BeamDev& b, const GridD
 // 547 -> 396 M warp instructions).  Also tried at 3 CTAs per SM: 4, 6 and 8
 // steps with the next group's loads issued before this one's sums, 8 and 12 steps,
 // and 64 registers (4 CTAs): all within 2%.
+// The integer pipe, half as wide as the float32 one, then bound the issue (64%
+// against 34% busy): steps left are counted in float32, their test and the
+// smallest t are three-operand minima, the index advances by multiply-adds.
+// Prologues: 32 beams at 128^3 334 -> 306 us, seven at 192^3 328 -> 295, 64 mixed
+// 2055 -> 1862, nine MLC beams 904 -> 872, 150 x 130 x 92 108 -> 98.
 constexpr int DDA_UNROLL = 5;
 
 __device__ float radiological_depth(const float* __restrict__ rho, const GridDev& g, int x, int y, int z,
@@ -582,25 +587,29 @@ __device__ float radiological_depth(const float* __restrict__ rho, const GridDev
   int idx = g.swap_xy ? (y * n0 + x) * n2 + z : (x * n1 + y) * n2 + z;
   const int dx = s0 * st0, dy = s1 * st1, dz = s2;
   // steps each axis may still take before the walk leaves the grid
-  int left0 = s0 > 0 ? n0 - 1 - x : x, left1 = s1 > 0 ? n1 - 1 - y : y, left2 = s2 > 0 ? n2 - 1 - z : z;
+  float left0 = (float)(s0 > 0 ? n0 - 1 - x : x), left1 = (float)(s1 > 0 ? n1 - 1 - y : y);
+  float left2 = (float)(s2 > 0 ? n2 - 1 - z : z);
+  auto inside = [&] { return fminf(fminf(left0, left1), left2) >= 0.0f; };
+  int one = 1;
+  asm volatile("" : "+r"(one));
   float deff = 0.0f, tprev = 0.0f;   // the first step adds rho * (t - 0), i.e. rho * t exactly
   // steps left are all >= 0 while the walk is inside the grid; an axis below 0
   // stays there.  A step past the exit reads no density and adds 0 * dt.
+  // The axis with the smallest t steps, z before y before x where they tie.
+  // one: 1 that the compiler does not know, so that the index sums are
+  // multiply-adds (the float32 pipe) and not integer sums
   auto steps = [&](float (&r)[DDA_UNROLL], float (&tv)[DDA_UNROLL]) {
 #pragma unroll
     for (int q = 0; q < DDA_UNROLL; ++q) {
-      r[q] = (left0 | left1 | left2) >= 0 ? __ldg(rho + idx) : 0.0f;
-      // the axis with the smallest t; z before y before x where they tie
-      const float t01 = fminf(t0, t1);
-      const bool a2 = t2 <= t01, a1 = !a2 && t1 <= t0, a0 = !a2 && !(t1 <= t0);
-      tv[q] = fminf(t01, t2);
-      if (a0) t0 = fadd(t0, d0);
-      if (a1) t1 = fadd(t1, d1);
-      if (a2) t2 = fadd(t2, d2);
-      idx += a2 ? dz : (a1 ? dy : dx);
-      left0 -= a0 ? 1 : 0;
-      left1 -= a1 ? 1 : 0;
-      left2 -= a2 ? 1 : 0;
+      r[q] = inside() ? __ldg(rho + idx) : 0.0f;
+      const float t = fminf(fminf(t0, t1), t2);
+      tv[q] = t;
+      asm("{\n .reg .pred p0, p1, p2;\n setp.le.f32 p2, %2, %7;\n setp.le.and.f32 p1|p0, %1, %7, !p2;\n"
+          " @p0 add.rn.f32 %0, %0, %8;\n @p1 add.rn.f32 %1, %1, %9;\n @p2 add.rn.f32 %2, %2, %10;\n"
+          " @p0 add.rn.f32 %3, %3, 0fBF800000;\n @p1 add.rn.f32 %4, %4, 0fBF800000;\n @p2 add.rn.f32 %5, %5, 0fBF800000;\n"
+          " @p0 mad.lo.s32 %6, %14, %11, %6;\n @p1 mad.lo.s32 %6, %14, %12, %6;\n @p2 mad.lo.s32 %6, %14, %13, %6;\n}"
+          : "+f"(t0), "+f"(t1), "+f"(t2), "+f"(left0), "+f"(left1), "+f"(left2), "+r"(idx)
+          : "f"(t), "f"(d0), "f"(d1), "f"(d2), "r"(dx), "r"(dy), "r"(dz), "r"(one));
     }
   };
   auto add = [&](const float (&r)[DDA_UNROLL], const float (&tv)[DDA_UNROLL]) {
@@ -610,7 +619,7 @@ __device__ float radiological_depth(const float* __restrict__ rho, const GridDev
       tprev = tv[q];
     }
   };
-  while ((left0 | left1 | left2) >= 0) {
+  while (inside()) {
     float r[DDA_UNROLL], tv[DDA_UNROLL];
     steps(r, tv);
     add(r, tv);
