@@ -1280,7 +1280,10 @@ __global__ void __launch_bounds__(ADJ_THREADS, 3) blocked_adjoint_kernel(const _
         if (n) atomicAdd(wbar + cur, gv * (double)n);
       }
     }
-    // byte fields: suffix sums over runs of lanes with the same beamlet, added by each run's first lane
+    // byte fields: suffix sums over runs of lanes with the same beamlet, added by each run's first lane.
+    // A lane without samples in a beamlet brings nothing to it, and a run without any adds nothing: the
+    // beamlet may lie off the grid, and a share that is not finite (a NaN in the dose gradient) times a
+    // count of 0 is not 0
     const int next_id = __shfl_down_sync(full, id0, 1);
     const unsigned same_next = __ballot_sync(full, lane < 31 && id0 == next_id);   // lane and lane + 1
     const int run = __clz(__brev(~(same_next >> lane)));           // lanes of the run after this one
@@ -1288,8 +1291,13 @@ __global__ void __launch_bounds__(ADJ_THREADS, 3) blocked_adjoint_kernel(const _
 #pragma unroll 1
     for (int f = 0; f < 4; ++f) {
       const float n = (float)((cnt >> (8 * f)) & 255u);
-      if (!__any_sync(full, n > 0.0f)) continue;
-      float hi = ghi * n, lo = __fmaf_rn(ghi, n, -hi) + glo * n;
+      const unsigned has = __ballot_sync(full, n > 0.0f);
+      if (!has) continue;
+      float hi = 0.0f, lo = 0.0f;
+      if (n > 0.0f) {
+        hi = ghi * n;
+        lo = __fmaf_rn(ghi, n, -hi) + glo * n;
+      }
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const float h2 = __shfl_down_sync(full, hi, o), l2 = __shfl_down_sync(full, lo, o);
@@ -1300,7 +1308,8 @@ __global__ void __launch_bounds__(ADJ_THREADS, 3) blocked_adjoint_kernel(const _
         }
       }
       const double sum = fabsf(hi) <= 3.4028234e38f ? (double)hi + (double)lo : (double)hi;
-      if (first && sum != 0.0) atomicAdd(wbar + id0 + (f >> 1) * bl.cols + (f & 1), sum);
+      const bool any = ((has >> lane) & ((2u << run) - 1u)) != 0;    // in this lane or the run's after it
+      if (first && any && sum != 0.0) atomicAdd(wbar + id0 + (f >> 1) * bl.cols + (f & 1), sum);
     }
   }
   if (__any_sync(full, bad) && lane == 0) atomicOr(flags, FLAG_PARALLEL_RAY);
