@@ -236,6 +236,11 @@ struct BeamletDev {
   int rows, cols, cell_rows, cell_cols, r0, c0;
 };
 
+// Chunks of 32 entries (one per lane) of a list.  Lists hold up to 2^31 - 1
+// voxels, so entry numbers rounded up to a launch's stride pass 2^31: they are
+// unsigned and compared as such.
+__host__ __device__ __forceinline__ int list_chunks(int count) { return (int)(((unsigned)count + 31u) >> 5); }
+
 struct Inter {
   double* blocked;
   float *d_eff, *oad, *fluence, *f_soften, *f_horn, *terma;

@@ -930,14 +930,14 @@ __device__ __forceinline__ bool terma_voxel(const float* __restrict__ rho, const
 template <bool EXACT>
 __device__ __forceinline__ void terma_entry(const float* __restrict__ rho, const GridDev& g, const BeamDev& b,
                                             const SettingsDev& s, float* __restrict__ T, const Inter& inter,
-                                            int all_voxels, int count, int e, const int* __restrict__ list_v,
+                                            int all_voxels, int count, unsigned e, const int* __restrict__ list_v,
                                             int* __restrict__ aabb, int* __restrict__ flags) {
   {
-    const bool live = e < count;
+    const bool live = e < (unsigned)count;
     int x = 0, y = 0, z = 0, bad = 0;
     float Tv = 0.0f;
     if (live) {
-      const int v = EXACT && !list_v ? e : list_v[e];
+      const int v = EXACT && !list_v ? (int)e : list_v[e];
       z = v % g.n[2];
       const int r = v / g.n[2];
       y = r % g.n[1];
@@ -985,8 +985,8 @@ __device__ __forceinline__ void terma_body(const float* __restrict__ rho, const 
                                            const int* __restrict__ list_v, int* __restrict__ aabb,
                                            int* __restrict__ flags, int cta, int n_ctas) {
   const int count = list_v ? *list_count : g.n[0] * g.n[1] * g.n[2];
-  const int rounds = (count + blockDim.x * n_ctas - 1) / (blockDim.x * n_ctas);
-  for (int it = 0; it < rounds; ++it)
+  const unsigned stride = blockDim.x * n_ctas, rounds = ((unsigned)count + stride - 1) / stride;
+  for (unsigned it = 0; it < rounds; ++it)
     terma_entry<true>(rho, g, b, s, T, inter, all_voxels, count, (it * n_ctas + cta) * blockDim.x + threadIdx.x,
                 list_v, aabb, flags);
 }
@@ -1027,7 +1027,7 @@ __global__ void __launch_bounds__(256, 3) terma_batch_kernel(const PrologueBeam*
     // chunks of beam b: ceil(list count / 32); the counts were written by the cull launch
     while (beam < n_beams) {
       count = recs[beam].aabb[6];
-      const int chunks = (count + 31) >> 5;
+      const int chunks = list_chunks(count);
       if (c < base + chunks) break;
       base += chunks;
       ++beam;
@@ -1185,12 +1185,11 @@ __global__ void __launch_bounds__(ADJ_THREADS, 3) blocked_adjoint_kernel(const _
   const float u0 = (float)(bl.r0 - 1999), w0 = (float)(bl.c0 - 1999);
   // the grid ends where the map does: its last row and column are read by the wrapped index only
   const bool whole = bl.r0 + bl.rows * bl.cell_rows <= 3999 && bl.c0 + bl.cols * bl.cell_cols <= 3999;
-  const int stride = gridDim.x * blockDim.x;
-  const int rounds = (count + stride - 1) / stride;
-  for (int it = 0; it < rounds; ++it) {
-    const int e = it * stride + blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned stride = gridDim.x * blockDim.x, rounds = ((unsigned)count + stride - 1) / stride;
+  for (unsigned it = 0; it < rounds; ++it) {
+    const unsigned e = it * stride + blockIdx.x * blockDim.x + threadIdx.x;
     float t = 0.0f, tb = 0.0f, pos[3] = {0.0f, 0.0f, 0.0f};
-    if (e < count) {
+    if (e < (unsigned)count) {
       const int v = list_v[e];
       const int z = v % g.n[2];
       const int r = v / g.n[2];

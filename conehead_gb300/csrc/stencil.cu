@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(256) scatter_radiological_kernel(
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
-  const int count = *list_count, chunks = (count + 31) >> 5;
+  const int count = *list_count, chunks = list_chunks(count);
   const int groups = (n_dirs + RADIO_GROUP - 1) / RADIO_GROUP;
   // density index of (x, y, z): steps along x and y as the reference reads them
   const int rx = swap_xy ? n2 : n1 * n2, ry = swap_xy ? n0 * n2 : n2;
