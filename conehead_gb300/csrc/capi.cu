@@ -128,7 +128,6 @@ struct ch_plan {
   int live_batches = 0;      // captured batches reading this plan's stencils
   long long wait_limit = 0;  // gather pipeline waits (try_wait iterations); 0 = MBAR_LIMIT
   int withhold = 0;          // test hook of the expired-wait path (ch_plan_set_wait_limit)
-  int* h_flags = nullptr;    // pinned copy of the counters (ch_plan_sync, ch_batch_sync)
   int epoch = 0;             // of the last call with the one-launch prologue
   bool flags_by_epoch = false;   // the last call reports failures in counters[6] == epoch, not in counters[1]
   int reweights = 0;         // spectrum switches served by reweighting the stencils
@@ -160,7 +159,6 @@ struct ch_plan {
   bool rec_pending[2] = {false, false};
   int rec_next = 0;
   ~ch_plan() {
-    if (h_flags) cudaFreeHost(h_flags);
     for (int i = 0; i < 2; ++i)
       if (rec_pending[i] && ev_rec[i]) cudaEventSynchronize(ev_rec[i]);
     spec.clear();
@@ -1951,15 +1949,16 @@ ch_status ch_dose_adjoint(ch_plan* P, const ch_grid* grid, const float* rho, int
   return CH_OK;
 }
 
-// Waits for `stream` and reports what its kernels left in `counters`: one copy
-// behind them into pinned memory and one wait (a wait and then a blocking copy
-// were two round trips).
+// Waits for `stream` and reports what its kernels left in `counters`.  The copy
+// goes to this call's own memory: threads may wait for batches of one plan at
+// the same time.  Queued on the stream, it costs one wait for both (a wait and
+// then a blocking copy were two round trips).
 namespace {
 ch_status read_flags(ch_plan* P, const void* counters, cudaStream_t s, bool by_epoch) {
-  if (!P->h_flags) CH_CUDA(cudaMallocHost(&P->h_flags, 8 * sizeof(int)));
-  CH_CUDA(cudaMemcpyAsync(P->h_flags, counters, 8 * sizeof(int), cudaMemcpyDeviceToHost, s));
-  CH_CUDA(cudaStreamSynchronize(s));
-  const int* c = P->h_flags;
+  int c[8] = {0};
+  const cudaError_t e = cudaMemcpyAsync(c, counters, sizeof(c), cudaMemcpyDeviceToHost, s);
+  CH_CUDA(cudaStreamSynchronize(s));   // also where the copy was refused: c must not be written later
+  CH_CUDA(e);
   const int flags = by_epoch ? (c[6] == P->epoch ? FLAG_PARALLEL_RAY : 0) : c[1];
   if (flags & FLAG_TIMEOUT) return fail(CH_ERR_TIMEOUT, "a bounded device wait expired in the cone stage");
   if (flags & FLAG_PARALLEL_RAY) return fail(CH_ERR_PARALLEL_RAY, "no intersection or line is within plane");
