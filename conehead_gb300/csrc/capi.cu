@@ -149,6 +149,7 @@ struct ch_plan {
   cudaStream_t last_stream = nullptr;
   ch_stats stats{};
   bool stats_pending = false;
+  bool stats_updates = false;    // counters[2..3] belong to the last call (the one-launch prologue resets none)
   bool timed = false;
   // pinned staging of the per-beam launch records, double buffered, so
   // their upload is a true async copy; ev_rec[i] marks when the upload from
@@ -1357,11 +1358,13 @@ ch_status run_group(ch_plan* P, int n, const ch_grid* grids, const float* const*
   P->stats = ch_stats{};
   P->stats.n_unique_dirs = B.U;
   P->stats_pending = true;
+  P->stats_updates = true;
   P->last_stream = s;
   P->flags_by_epoch = false;
   if (B.spectral && !scatter && !inter && fused_prologue(B)) {
     P->epoch += 1;
     P->flags_by_epoch = true;
+    P->stats_updates = false;
     const std::vector<PrologueBeam> pb = make_prologue_records(B, S);
     FusedRecords rec;
     std::memcpy(rec.r, pb.data(), pb.size() * sizeof(PrologueBeam));
@@ -2223,11 +2226,13 @@ ch_status ch_plan_stats(ch_plan* P, ch_stats* out) {
     CH_CUDA(cudaEventElapsedTime(&P->stats.ms_prologue, P->ev[0], P->ev[1]));
     CH_CUDA(cudaEventElapsedTime(&P->stats.ms_range, P->ev[1], P->ev[2]));
     CH_CUDA(cudaEventElapsedTime(&P->stats.ms_cone, P->ev[2], P->ev[3]));
-    int c[4];
-    CH_CUDA(cudaMemcpy(c, P->counters.p, sizeof(c), cudaMemcpyDeviceToHost));
-    unsigned long long u;
-    std::memcpy(&u, c + 2, sizeof(u));
-    P->stats.updates = (double)u;
+    if (P->stats_updates) {
+      int c[4];
+      CH_CUDA(cudaMemcpy(c, P->counters.p, sizeof(c), cudaMemcpyDeviceToHost));
+      unsigned long long u;
+      std::memcpy(&u, c + 2, sizeof(u));
+      P->stats.updates = (double)u;
+    }
     P->stats_pending = false;
   }
   *out = P->stats;

@@ -3,6 +3,7 @@ go with it.
 
 * Captured batches of one plan, waited for by two threads at the same time, each
   report their own failure.
+* Statistics are the last call's, whatever method the call before it used.
 """
 import threading
 
@@ -68,3 +69,21 @@ def test_two_threads_wait_for_batches_of_one_plan(settings):
     for t in threads:
         t.join()
     assert wrong == [0, 0]
+
+
+@pytest.mark.parametrize("n", [12, 100])    # the one-launch prologue, the list
+def test_statistics_after_a_method_switch(settings, n):
+    eng = _engine(settings)
+    job = _job(eng, settings, n=n)
+    for _ in range(2):
+        eng.set_tuning(cone_method=1)
+        eng.run(job)
+        eng.sync()
+        gather = eng.stats()
+        assert gather["updates"] > 0 and gather["n_units"] > 0
+        eng.set_tuning(cone_method=0)
+        eng.run(job)
+        eng.sync()
+        spectral = eng.stats()
+        assert spectral["updates"] == 0 and spectral["n_units"] == 0
+        assert spectral["ms_prologue"] > 0 and spectral["ms_cone"] > 0
