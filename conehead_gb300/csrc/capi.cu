@@ -121,6 +121,11 @@ struct SpecEntry {
   ~SpecEntry() { shat.release(); }
 };
 
+// Failures are reported in counters[1], which launches with a list reset, and
+// those of the one-launch prologue (parallel rays) in counters[6], which then
+// holds the call's epoch.
+constexpr int FLAGS_RESET = 1, FLAGS_EPOCH = 2;
+
 struct ch_plan {
   int device = 0;
   int n_sm = 0;
@@ -128,8 +133,9 @@ struct ch_plan {
   int live_batches = 0;      // captured batches reading this plan's stencils
   long long wait_limit = 0;  // gather pipeline waits (try_wait iterations); 0 = MBAR_LIMIT
   int withhold = 0;          // test hook of the expired-wait path (ch_plan_set_wait_limit)
-  int epoch = 0;             // of the last call with the one-launch prologue
-  bool flags_by_epoch = false;   // the last call reports failures in counters[6] == epoch, not in counters[1]
+  int epoch = 0;             // of the last dose call
+  bool new_call = false;     // no group of the current dose call has been launched yet
+  int flag_words = 0;        // where the last call's launches report failures (FLAGS_*)
   int reweights = 0;         // spectrum switches served by reweighting the stencils
   std::vector<std::unique_ptr<FrameStencils>> frames;   // beam-frame cone stencils by orientation
   uint64_t use_clock = 0;
@@ -1293,13 +1299,14 @@ bool fused_prologue(const BatchPlan& B) {
 // prologues, dose zeroing, tap ranges, one persistent gather.  Only kernel
 // launches and memsets, so it can be captured into a CUDA graph.  ev (4
 // events, or NULL) marks the stage boundaries.
+// keep: the counters that hold failures of the same call's earlier launches.
 ch_status enqueue_batch(ch_plan* P, const BatchPlan& B, const Scratch& S, const ch_intermediates* inter,
-                        const cudaEvent_t* ev, cudaStream_t s) {
+                        const cudaEvent_t* ev, cudaStream_t s, unsigned keep = 0) {
   const int n = (int)B.jobs.size();
   int* flags = S.counters + 1;
   unsigned long long* updates = reinterpret_cast<unsigned long long*>(S.counters + 2);
   if (ev) CH_CUDA(cudaEventRecord(ev[0], s));
-  launch_init_scratch(S.aabb, n, S.counters, s);
+  launch_init_scratch(S.aabb, n, S.counters, s, keep);
   if (inter) {
     // intermediates wanted: the per-beam prologue writes them
     for (int i = 0; i < n; ++i) {
@@ -1360,10 +1367,13 @@ ch_status run_group(ch_plan* P, int n, const ch_grid* grids, const float* const*
   P->stats_pending = true;
   P->stats_updates = true;
   P->last_stream = s;
-  P->flags_by_epoch = false;
-  if (B.spectral && !scatter && !inter && fused_prologue(B)) {
+  if (P->new_call) {          // (a refused call leaves the failures of the one before it to be read)
+    P->new_call = false;
     P->epoch += 1;
-    P->flags_by_epoch = true;
+    P->flag_words = 0;
+  }
+  if (B.spectral && !scatter && !inter && fused_prologue(B)) {
+    P->flag_words |= FLAGS_EPOCH;
     P->stats_updates = false;
     const std::vector<PrologueBeam> pb = make_prologue_records(B, S);
     FusedRecords rec;
@@ -1376,11 +1386,13 @@ ch_status run_group(ch_plan* P, int n, const ch_grid* grids, const float* const*
     CH_CUDA(cudaEventRecord(P->ev[1], s));
     return enqueue_spectral(P, B, S, false, P->ev, s);
   }
+  const unsigned keep = ((P->flag_words & FLAGS_RESET) ? 1u << 1 : 0u) | ((P->flag_words & FLAGS_EPOCH) ? 1u << 6 : 0u);
+  P->flag_words |= FLAGS_RESET;
   if (scatter) {
     // plain path: prologues, then one per-voxel scatter launch per beam
     int* flags = S.counters + 1;
     CH_CUDA(cudaEventRecord(P->ev[0], s));
-    launch_init_scratch(S.aabb, n, S.counters, s);
+    launch_init_scratch(S.aabb, n, S.counters, s, keep);
     for (int i = 0; i < n; ++i) {
       const BeamJob& J = B.jobs[i];
       int all = 0;
@@ -1418,19 +1430,20 @@ ch_status run_group(ch_plan* P, int n, const ch_grid* grids, const float* const*
     segs.push_back(Seg{S.range_beams, rb.data(), rb.size() * sizeof(RangeBeam)});
   }
   if (!segs.empty() && (st = stage_records(P, segs, s)) != CH_OK) return st;
-  if ((st = enqueue_batch(P, B, S, inter, P->ev, s)) != CH_OK) return st;
+  if ((st = enqueue_batch(P, B, S, inter, P->ev, s, keep)) != CH_OK) return st;
   P->stats.n_units = B.spectral ? 0 : B.total_units;
   return CH_OK;
 }
 
 // Beams with physics options run one at a time, each with its own stencils
 // (beam-frame cones) and path (radiological distance: the scatter); plain
-// beams keep the fused batch.
+// beams keep the fused batch.  A failure of any of them is the call's.
 ch_status run(ch_plan* P, int n, const ch_grid* grids, const float* const* rho, const int* swap_xy,
               const ch_beam* beams, const ch_settings* settings, float* const* dose, const ch_intermediates* inter,
               bool scatter, cudaStream_t s) {
   bool any = false;
   for (int i = 0; i < n && settings && beams; ++i) any |= settings[i].options != 0;
+  if (P) P->new_call = true;
   if (!any) return run_group(P, n, grids, rho, swap_xy, beams, settings, dose, inter, scatter, false, nullptr, s);
   if (!P) return fail(CH_ERR_INVALID_ARG, "plan is NULL");
   if (!P->have_kernel) return fail(CH_ERR_NO_KERNEL, "ch_plan_set_kernel has not been called");
@@ -1678,7 +1691,7 @@ ch_status ch_dose_static(ch_plan* P, const ch_grid* grid, const float* rho, int 
   // rather than an earlier call's timings
   P->stats_pending = false;
   P->stats = ch_stats{};
-  P->flags_by_epoch = false;
+  P->flag_words = FLAGS_RESET;
   // aabb and the list count must start from their reset values; TERMA is
   // rewritten in full by the prologue and the range tables by range_kernel
   launch_init_scratch(aabb, 1, counters, s);
@@ -1863,7 +1876,7 @@ ch_status ch_cone(ch_plan* P, const ch_grid* grid, const float* in, float* out, 
   if ((st = ensure_stencils(P, grid->spacing, grid->n, s)) != CH_OK) return st;
   CH_CUDA(P->aabb.ensure(8 * sizeof(int)));
   CH_CUDA(P->counters.ensure(8 * sizeof(int)));
-  P->flags_by_epoch = false;
+  P->flag_words = FLAGS_RESET;
   launch_init_scratch(P->aabb.as<int>(), 1, P->counters.as<int>(), s);
   st = cone_operator(P, *grid, in, out, transpose != 0, P->aabb.as<int>(), nullptr, s);
   if (st != CH_OK) return st;
@@ -1915,7 +1928,7 @@ ch_status ch_dose_adjoint(ch_plan* P, const ch_grid* grid, const float* rho, int
   int* flags = counters + 1;
   const BeamDev b = make_beam(*beam, *grid, settings->samples);
   const SettingsDev sd = make_settings(*settings);
-  P->flags_by_epoch = false;
+  P->flag_words = FLAGS_RESET;
   launch_init_scratch(box, 2, counters, s);
   // forward prologue: TERMA, its box (gather) and the list of voxels the beam reaches
   const bool gather = !spec_batch(P, 1, grid);
@@ -1957,12 +1970,12 @@ ch_status ch_dose_adjoint(ch_plan* P, const ch_grid* grid, const float* rho, int
 // the same time.  Queued on the stream, it costs one wait for both (a wait and
 // then a blocking copy were two round trips).
 namespace {
-ch_status read_flags(ch_plan* P, const void* counters, cudaStream_t s, bool by_epoch) {
+ch_status read_flags(const void* counters, cudaStream_t s, int words, int epoch) {
   int c[8] = {0};
   const cudaError_t e = cudaMemcpyAsync(c, counters, sizeof(c), cudaMemcpyDeviceToHost, s);
   CH_CUDA(cudaStreamSynchronize(s));   // also where the copy was refused: c must not be written later
   CH_CUDA(e);
-  const int flags = by_epoch ? (c[6] == P->epoch ? FLAG_PARALLEL_RAY : 0) : c[1];
+  const int flags = ((words & FLAGS_RESET) ? c[1] : 0) | (((words & FLAGS_EPOCH) && c[6] == epoch) ? FLAG_PARALLEL_RAY : 0);
   if (flags & FLAG_TIMEOUT) return fail(CH_ERR_TIMEOUT, "a bounded device wait expired in the cone stage");
   if (flags & FLAG_PARALLEL_RAY) return fail(CH_ERR_PARALLEL_RAY, "no intersection or line is within plane");
   return CH_OK;
@@ -2057,7 +2070,7 @@ ch_status ch_batch_launch(ch_batch* bt, void* stream) {
 ch_status ch_batch_sync(ch_batch* bt, void* stream) {
   if (!bt) return fail(CH_ERR_INVALID_ARG, "batch is NULL");
   CH_CUDA(cudaSetDevice(bt->P->device));
-  return read_flags(bt->P, bt->counters.p, (cudaStream_t)stream, false);
+  return read_flags(bt->counters.p, (cudaStream_t)stream, FLAGS_RESET, 0);
 }
 
 void ch_batch_destroy(ch_batch* bt) {
@@ -2215,7 +2228,7 @@ ch_status ch_plan_sync(ch_plan* P, void* stream) {
     CH_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
     return CH_OK;
   }
-  return read_flags(P, P->counters.p, (cudaStream_t)stream, P->flags_by_epoch);
+  return read_flags(P->counters.p, (cudaStream_t)stream, P->flag_words, P->epoch);
 }
 
 ch_status ch_plan_stats(ch_plan* P, ch_stats* out) {

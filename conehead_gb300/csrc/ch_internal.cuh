@@ -435,7 +435,8 @@ cudaError_t setup_cone_kernel();
 void launch_range(const RangeBeam* rbs_dev, int n_beams, int max_tiles, const ConeDirs& D, cudaStream_t st);
 void launch_gather(const ConeBeam* beams_dev, int n_beams, const ConeDirs& D, int total_units, int n_ctas,
                    int* unit_counter, unsigned long long* updates, int* flags, cudaStream_t st);
-void launch_init_scratch(int* aabb, int n_beams, int* counters, cudaStream_t st);
+// keep: a bit per counter that is not reset
+void launch_init_scratch(int* aabb, int n_beams, int* counters, cudaStream_t st, unsigned keep = 0);
 void launch_mlc_raster(const ch_mlc& m, float* out, int rows, int cols, int r0, int c0, cudaStream_t st);
 void launch_nonzero_box(const float* x, int n0, int n1, int n2, int* box, cudaStream_t st);
 void launch_beamlet_fill(const float* w, const BeamletDev& bl, float* crop, cudaStream_t st);

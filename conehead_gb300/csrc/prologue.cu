@@ -1374,16 +1374,16 @@ void launch_prologue_batch(const PrologueBeam* recs, int n_beams, long long max_
                flags, work);
 }
 
-__global__ void init_scratch_kernel(int* aabb, int n_beams, int* counters) {
+__global__ void init_scratch_kernel(int* aabb, int n_beams, int* counters, unsigned keep) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   // per beam: lo/hi pairs of the TERMA box, then the prologue list count
   if (i < n_beams * 8) aabb[i] = (i % 8 >= 6) ? 0 : ((i % 2 == 0) ? INT_MAX : INT_MIN);
-  if (i < 8) counters[i] = 0;
+  if (i < 8 && !((keep >> i) & 1u)) counters[i] = 0;
 }
 
-void launch_init_scratch(int* aabb, int n_beams, int* counters, cudaStream_t st) {
+void launch_init_scratch(int* aabb, int n_beams, int* counters, cudaStream_t st, unsigned keep) {
   const int n = n_beams * 8 > 8 ? n_beams * 8 : 8;
-  init_scratch_kernel<<<(n + 255) / 256, 256, 0, st>>>(aabb, n_beams, counters);
+  init_scratch_kernel<<<(n + 255) / 256, 256, 0, st>>>(aabb, n_beams, counters, keep);
 }
 
 }  // namespace ch

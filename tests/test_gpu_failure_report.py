@@ -3,6 +3,8 @@ go with it.
 
 * Captured batches of one plan, waited for by two threads at the same time, each
   report their own failure.
+* A call of several beams fails where any of them does, whatever launches it
+  takes for each; the next call does not, and a refused call reports nothing.
 * Statistics are the last call's, whatever method the call before it used.
 """
 import threading
@@ -87,3 +89,34 @@ def test_statistics_after_a_method_switch(settings, n):
         spectral = eng.stats()
         assert spectral["updates"] == 0 and spectral["n_units"] == 0
         assert spectral["ms_prologue"] > 0 and spectral["ms_cone"] > 0
+
+
+# geometric beams in the room frame take the one-launch prologue, the others a list
+KINDS = ({}, {"coneFrame": "beam"}, {"coneDistance": "radiological"})
+
+
+@pytest.mark.parametrize("first", range(3))
+@pytest.mark.parametrize("second", range(3))
+def test_any_beam_of_a_call_may_fail(settings, first, second):
+    eng = _engine(settings)
+    options = [dict(settings, **KINDS[k]) for k in (first, second)]
+    # a beam with options makes the call run beam by beam
+    last = _job(eng, dict(settings, **KINDS[1]), n=9)
+    for bad in (None, 0, 1):
+        jobs = [_job(eng, o, parallel=(i == bad)) for i, o in enumerate(options)] + [last]
+        eng.run_batch(jobs)
+        if bad is None:
+            eng.sync()
+            continue
+        for _ in range(2):
+            with pytest.raises(RuntimeError, match="plane"):
+                eng.sync()
+        broken = _job(eng, settings)
+        broken.grid.n[0] = 0
+        with pytest.raises(Exception, match="invalid argument"):
+            eng.run(broken)
+        with pytest.raises(RuntimeError, match="plane"):
+            eng.sync()
+        for o in options:
+            eng.run(_job(eng, o))
+            eng.sync()
