@@ -24,7 +24,11 @@
 
 namespace ch {
 
-constexpr float SAMPLE_DELTA = 0.05f;   // cells (0.1 mm) of float32 slack
+constexpr float SAMPLE_DELTA = 0.05f;   // cells (0.1 mm) of float32 slack of the general paths
+// largest bound of a lattice sample's cell coordinates with which one neighbour
+// per axis, on the sample's side of its cell, is all it may fall in (a bound
+// below half a cell, less the roundings of the test)
+constexpr float LATTICE_DELTA_MAX = 0.25f;
 
 // partial sums 0, 1/27, 1/27+1/27, ... accumulated in float64 as the
 // reference does for a block value of exactly 1.0 and 3x3x3 samples
@@ -214,15 +218,19 @@ __device__ __forceinline__ float sample_value(const BeamDev& b, const GridDev& g
   return v;
 }
 
-// General blocked fraction: any sample count, float32 source arrays, or
-// transmission values other than 0 and 1 (float64, reference order
-// acc = acc + v / S^3 over ix, iy, iz).
+// Whether the general paths must mirror every sample of a voxel: their fixed
+// slack covers the float32 projection only where lattice_centre's bound, of the
+// same terms in another order, is known and below half of it.
+__device__ __noinline__ bool general_exact(const BeamDev& b, const float* pos);
+
+// General blocked fraction, where the lattice below does not hold (float64,
+// reference order acc = acc + v / S^3 over ix, iy, iz).
 __device__ __noinline__ double blocked_general(const BeamDev& b, const GridDev& g, int S, const float* pos,
                                                int& bad) {
   float off[3];
   // f32(f64(s) / S) == fdiv(s, S): double rounding is innocuous for float32 operands
   for (int k = 0; k < 3; ++k) off[k] = fdiv(g.spacing[k], (float)S);
-  const bool exact_all = b.geom_f32 != 0;
+  const bool exact_all = general_exact(b, pos);
   double acc = 0.0;
   const double denom = (double)S * (double)S * (double)S;
   float last_v = -1.0f;
@@ -266,7 +274,8 @@ struct Centre {
 //   |d(K x0 / nd)| <= |K| (B + |x0 / nd| A) / (|nd| - A).
 // False when a sub-sample may lie closer to the source plane than 0.2 |K| or
 // may read the wrapped cell -2000 of a crop that holds the map's last row or
-// column: those voxels, and float32 source arrays, take blocked_general.
+// column, or where delta is too large for a map's neighbour test: those voxels,
+// and float32 source arrays, take blocked_general.
 //
 // delta bounds the difference between a float32 cell coordinate and the
 // reference's, whose ray and plane point are float32 stores as well.  With
@@ -295,7 +304,15 @@ __device__ __forceinline__ bool lattice_centre(const BeamDev& b, const float* po
   c.delta = mag * (b.err_x + (fmaxf(l0, l2) + 0.01f) * b.err_n) + 0.002f;
   c.mu = mag * (b.lat_0 + l0 * b.lat_n) + c.delta;
   c.mw = mag * (b.lat_2 + l2 * b.lat_n) + c.delta;
+  if (!b.uniform && !(c.delta <= LATTICE_DELTA_MAX)) return false;
   return !b.wraps || (c.u - c.mu > -1999.0f && c.w - c.mw > -1999.0f);
+}
+
+__device__ __noinline__ bool general_exact(const BeamDev& b, const float* pos) {
+  Centre c;
+  c.delta = 1.0e30f;
+  lattice_centre(b, pos, c);       // leaves delta alone near the source plane and for float32 sources
+  return !(c.delta <= 0.5f * SAMPLE_DELTA);
 }
 
 // Calls f(ix, iy, iz, u, w) for every sub-sample in the reference's order.  Rolled:
@@ -1104,12 +1121,14 @@ __device__ __forceinline__ int beamlet_of(const BeamDev& b, const BeamletDev& bl
 }
 
 // Beamlet of sub-sample (ix, iy, iz): the float32 projection decides when
-// every cell within SAMPLE_DELTA of it lies in one beamlet, otherwise the
-// exact float64 mirror finds the reference's cell.  (The forward pass may
+// every cell within SAMPLE_DELTA of it lies in one beamlet, otherwise (or
+// where exact says that the bound may not hold) the exact float64 mirror finds
+// the reference's cell.  (The forward pass may
 // settle a sample on value alone; the derivative needs the beamlet.)
 __device__ int sample_beamlet(const BeamDev& b, const BeamletDev& bl, const GridDev& g, const float* pos,
-                              const float* off, float rx, float ry, float rz, int ix, int iy, int iz, int& bad) {
-  if (!b.geom_f32) {
+                              const float* off, float rx, float ry, float rz, int ix, int iy, int iz, bool exact,
+                              int& bad) {
+  if (!b.geom_f32 && !exact) {
     const float p0 = pos[0] + rx, p1 = pos[1] + ry, p2 = pos[2] + rz;
     const float np_ = b.vyf[0] * p0 + b.vyf[1] * p1 + b.vyf[2] * p2;
     const float m0p = b.m0f[0] * p0 + b.m0f[1] * p1 + b.m0f[2] * p2;
@@ -1267,13 +1286,14 @@ __global__ void __launch_bounds__(ADJ_THREADS, 3) blocked_adjoint_kernel(const _
             sample(id);
           });
         } else {
+          const bool exact = general_exact(b, pos);
           for (int ix = 0; ix < S; ++ix)
             for (int iy = 0; iy < S; ++iy)
               for (int iz = 0; iz < S; ++iz) {
                 const float rx = off[0] * ((float)ix + 0.5f) - g.spacing[0] * 0.5f;
                 const float ry = off[1] * ((float)iy + 0.5f) - g.spacing[1] * 0.5f;
                 const float rz = off[2] * ((float)iz + 0.5f) - g.spacing[2] * 0.5f;
-                sample(sample_beamlet(b, bl, g, pos, off, rx, ry, rz, ix, iy, iz, bad));
+                sample(sample_beamlet(b, bl, g, pos, off, rx, ry, rz, ix, iy, iz, exact, bad));
               }
         }
         if (n) atomicAdd(wbar + cur, gv * (double)n);
