@@ -698,21 +698,31 @@ BeamDev make_beam(const ch_beam& in, const ch_grid& g, int samples) {
   b.vyw = (b.vy[0] * w0 + b.vy[1] * w1) + b.vy[2] * w2;
   b.vywf = (b.vyf[0] * b.srcf[0] + b.vyf[1] * b.srcf[1]) + b.vyf[2] * b.srcf[2];
   b.geom_f32 = in.geom_f32;
+  // Pairs (project_pairs) wherever nothing overflows.  Small entries lose nothing:
+  // what underflows of a product is below 2^-140, the denominator is above 1e-6
+  // and the projections enter squares.  (Sines of right angles are 6e-17 and
+  // their products 4e-33; a lower bound of 1e-12 left gantries 0, 180 and 270 out:
+  // prologue of 32 beams at 128^3, gantry 0, 305 us in float64, 243 in pairs.)
   b.pairs = in.geom_f32 ? 0 : 1;
-  auto low = [&](double v, double lo, double hi) {   // its low part; |v| is 0 or in [lo, hi]
-    const double a = std::fabs(v);
-    if (!(a == 0.0 || (a >= lo && a <= hi))) b.pairs = 0;
-    return (float)(v - (double)(float)v);
+  auto bound = [&](double v, double most) {
+    if (!(std::fabs(v) <= most)) b.pairs = 0;
   };
+  auto low = [](double v) { return (float)(v - (double)(float)v); };   // the part beside float32(v)
   for (int k = 0; k < 3; ++k) {
-    b.srcl[k] = low(in.src[k], 1e-12, 1e6);
-    b.vyl[k] = low(b.vy[k], 1e-18, 1e3);
-    b.m0l[k] = low(b.m0[k], 1e-18, 1e3);
-    b.m2l[k] = low(b.m2[k], 1e-18, 1e3);
-    if (!(std::fabs((double)g.origin[k]) <= 1e6 && (double)g.n[k] * g.spacing[k] <= 1e6)) b.pairs = 0;
+    bound(b.src[k], 1e6);
+    bound(b.vy[k], 1e3);
+    bound(b.m0[k], 1e3);
+    bound(b.m2[k], 1e3);
+    bound(g.origin[k], 1e6);
+    bound((double)g.n[k] * g.spacing[k], 1e6);
+    b.vyl[k] = low(b.vy[k]);
+    b.m0l[k] = low(b.m0[k]);
+    b.m2l[k] = low(b.m2[k]);
   }
+  bound(b.vyw, 1e9);
+  if (std::fabs(b.vyw) < 1e-12) b.pairs = 0;    // the quotient's scale
   b.vywh = (float)b.vyw;
-  b.vywl = low(b.vyw, 1e-12, 1e9);
+  b.vywl = low(b.vyw);
   const double nS = b.vy[0] * b.src[0] + b.vy[1] * b.src[1] + b.vy[2] * b.src[2];
   const double m0S = b.m0[0] * b.src[0] + b.m0[1] * b.src[1] + b.m0[2] * b.src[2];
   const double m2S = b.m2[0] * b.src[0] + b.m2[1] * b.src[1] + b.m2[2] * b.src[2];

@@ -95,9 +95,9 @@ struct BeamDev {
   double srcd[3];                       // float32(src)
   float srcf[3], vyf[3], m0f[3], m2f[3], vywf;  // float32 copies (geom_f32 path)
   int geom_f32;
-  // low parts of the float64 values beside srcf, vyf, m0f, m2f and vywh (project_pairs)
-  float srcl[3], vyl[3], m0l[3], m2l[3], vywh, vywl;
-  int pairs;                            // they hold 48 bits and no product over- or underflows
+  // low parts of the float64 values beside vyf, m0f, m2f and vywh (project_pairs)
+  float vyl[3], m0l[3], m2l[3], vywh, vywl;
+  int pairs;                            // no product of them overflows (make_beam)
   // fast approximate projection: xb ~ c0 + si * (m0.S - m0.p), si = K / (n.S - n.p)
   float a_c0, a_c2, a_m0S, a_m2S, a_nS, a_K;
   // cull box in beam coordinates (cm) for voxel centres (inclusive)
