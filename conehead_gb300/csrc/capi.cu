@@ -951,7 +951,7 @@ ch_status stage_records(ch_plan* P, const std::vector<Seg>& segs, cudaStream_t s
 
 // ------------------------------------------------- spectral cone layout --
 // Beams of one grid shape share a launch of up to SPEC_MAX_BEAMS, in call
-// order; the launches of a batch run one after another in one work arena (A and
+// order, as many as SPEC_WORK_MAX holds (at least one); the launches of a batch run one after another in one work arena (A and
 // B of each beam of the launch).
 struct SpecPlanBeam {
   int job;
@@ -966,6 +966,11 @@ struct SpecLayout {
   std::vector<SpecPlanLaunch> launches;
   size_t arena = 0;          // float2
 };
+
+// Work arena of a launch, in complex values (16 GiB).  A beam needs 0.2 GB at 201^3,
+// 0.4 at 256^3, 1.2 at 350^3, and a few of those fill the GPU.  Cone stage of 32 beams
+// without a bound / at 16 / at 8 GiB: 300^3 (26 GB) 85.9 / 86.1 / 86.3 ms, 256^3 (13 GB) 18.3 / 18.3 / 18.3.
+constexpr size_t SPEC_WORK_MAX = (size_t)2 << 30;
 
 constexpr long long kSpecMaxVolume = 1ll << 28;   // largest Mx My Mz (S^ of 2 GiB)
 
@@ -999,14 +1004,16 @@ SpecLayout spec_layout(int n, const ch_grid* grids) {
     const bool plane = spec_plane_path(M);
     const size_t a_sz = plane ? (size_t)M[2] * spec_plane_pitch(d) : (size_t)d[0] * d[1] * M[2];
     const size_t b_sz = plane ? 0 : (size_t)d[0] * M[1] * M[2];
-    for (size_t p = 0; p < group.size(); p += SPEC_MAX_BEAMS) {
+    const size_t per_beam = (a_sz + 31) / 32 * 32 + (b_sz + 31) / 32 * 32;
+    const size_t most = std::max<size_t>(1, std::min<size_t>(SPEC_MAX_BEAMS, SPEC_WORK_MAX / per_beam));
+    for (size_t p = 0; p < group.size(); p += most) {
       SpecPlanLaunch l;
       for (int k = 0; k < 3; ++k) {
         l.n[k] = d[k];
         l.M[k] = M[k];
       }
       size_t off = 0;
-      for (size_t q = p; q < std::min(group.size(), p + SPEC_MAX_BEAMS); ++q) {
+      for (size_t q = p; q < std::min(group.size(), p + most); ++q) {
         SpecPlanBeam b;
         b.job = group[q];
         b.a_off = off;
