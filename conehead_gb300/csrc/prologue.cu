@@ -567,6 +567,8 @@ __device__ __forceinline__ double blocked_fraction(const BeamDev& b, const GridD
     }
   });
   if (hi == 0.0f && lo == 0.0f && S == 3) return c_unit_partial[ones];
+  // past float32's range (or an infinity or NaN in the map) the float64 sum decides
+  if (!(fabsf(hi) <= 3.4028234e38f)) return blocked_general(b, g, S, pos, bad);
   return ddiv(dadd(dadd((double)hi, (double)lo), (double)ones), count);
 }
 
