@@ -9,6 +9,7 @@
 // beams' cost, 236 us at 432).
 #pragma once
 
+#include "ch_internal.cuh"
 #include "spectral_dft.cuh"
 
 namespace ch {

@@ -9,9 +9,12 @@
 // against float64 6.1e-8 -> 5.9e-8).  Cone stage, scalar / this: 64 mixed beams
 // 2768 / 2615 us, 32 at 128^3 1268 / 1205, four at 160^3 424 / 396, at 201^3 1271
 // / 1237, seven at 192^3 1254 / 1236.
+//
+// The header needs nothing but the vector types and compiles for the host too
+// (tests/test_spectral_dft_cpu.py), with scalar forms of the packed instructions.
 #pragma once
 
-#include "ch_internal.cuh"
+#include <cuda_runtime.h>
 
 namespace ch {
 
@@ -50,6 +53,7 @@ constexpr double ct_sin(int k, int n) {
 constexpr double ct_cos(int k, int n) { return ct_sin(4 * (k % n) + n, 4 * n); }
 
 // -------------------------------------------------------- packed pairs --
+#ifdef __CUDA_ARCH__
 __device__ __forceinline__ unsigned long long pack2(float x, float y) {
   unsigned long long r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
@@ -60,26 +64,43 @@ __device__ __forceinline__ float2 unpack2(unsigned long long r) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
   return a;
 }
+#endif
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) {
+#ifdef __CUDA_ARCH__
   unsigned long long r;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a.x, a.y)), "l"(pack2(b.x, b.y)));
   return unpack2(r);
+#else
+  return make_float2(a.x + b.x, a.y + b.y);
+#endif
 }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) {
+#ifdef __CUDA_ARCH__
   unsigned long long r;
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a.x, a.y)), "l"(pack2(b.x, b.y)));
   return unpack2(r);
+#else
+  return make_float2(a.x - b.x, a.y - b.y);
+#endif
 }
 __device__ __forceinline__ float2 cscale(float2 a, float k) {
+#ifdef __CUDA_ARCH__
   unsigned long long r;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a.x, a.y)), "l"(pack2(k, k)));
   return unpack2(r);
+#else
+  return make_float2(k * a.x, k * a.y);
+#endif
 }
 // k a + b
 __device__ __forceinline__ float2 cfma(float k, float2 a, float2 b) {
+#ifdef __CUDA_ARCH__
   unsigned long long r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pack2(a.x, a.y)), "l"(pack2(k, k)), "l"(pack2(b.x, b.y)));
   return unpack2(r);
+#else
+  return make_float2(__builtin_fmaf(k, a.x, b.x), __builtin_fmaf(k, a.y, b.y));
+#endif
 }
 // -+i (a - b)
 template <bool INV>
