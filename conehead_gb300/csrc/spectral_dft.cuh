@@ -4,8 +4,8 @@
 // (x pass of seven beams at 192^3: 0.32 ms of the pipe, 0.27 of memory, in 0.68).
 // So complex sums take one packed instruction (add.rn.f32x2: the pipe's time of
 // two, one issue slot, the same roundings), and the rotations inside 16 points
-// are two multiply-adds (x + t y, y - t x with t = tan 22.5 or 1) whose common
-// factor cos 22.5 or cos 45 joins the sums that follow (rms error of 16 points
+// are two multiply-adds (t x + y, t y - x with t = cot 22.5 or 1) whose common
+// factor sin 22.5 or cos 45 joins the sums that follow (rms error of 16 points
 // against float64 6.1e-8 -> 5.9e-8).  Cone stage, scalar / this: 64 mixed beams
 // 2768 / 2615 us, 32 at 128^3 1268 / 1205, four at 160^3 424 / 396, at 201^3 1271
 // / 1237, seven at 192^3 1254 / 1236.
@@ -134,24 +134,30 @@ __device__ __forceinline__ void dft4_scaled(float k, float2 s02, float2 d02, flo
   a3 = cfma(-k, mi, d02);
 }
 
-// v exp(-+i theta) by its common factor: 22.5 and 67.5 degrees / C1, 45 / R2
-constexpr float DFT_C1 = 0.92387953251128674f;   // cos(pi/8) = sin(3 pi/8)
-constexpr float DFT_T1 = 0.41421356237309505f;   // tan(pi/8) = cot(3 pi/8)
+// v exp(-+i theta) by its common factor: 22.5 and 67.5 degrees / S1, 45 / R2
+// (by sin 22.5 and not by cos 22.5: their roundings to float32, -1.6e-8 and -3.1e-8, are
+// the same in every butterfly, a gain that a dose passes six times and S^ three.
+// With this factor the rotations' gain cancels that of the 45 degrees, 5e-11 for
+// 16 points, where the other left -1.1e-8.  Error of a dose against 64 bits: 64^3
+// 1.69e-7 -> 1.29e-7, 128^3 2.34 -> 1.70, 150 x 130 x 92 2.95 -> 2.67, 192^3 2.63 ->
+// 2.05; the same instructions, the same times)
+constexpr float DFT_S1 = 0.38268343236508977f;   // sin(pi/8) = cos(3 pi/8)
+constexpr float DFT_T1 = 2.4142135623730950f;    // cot(pi/8) = tan(3 pi/8)
 constexpr float DFT_R2 = 0.70710678118654752f;   // cos(pi/4)
 template <bool INV>
 __device__ __forceinline__ float2 lift22(float2 v) {
-  return INV ? make_float2(v.x - DFT_T1 * v.y, v.y + DFT_T1 * v.x)
-             : make_float2(v.x + DFT_T1 * v.y, v.y - DFT_T1 * v.x);
+  return INV ? make_float2(DFT_T1 * v.x - v.y, DFT_T1 * v.y + v.x)
+             : make_float2(DFT_T1 * v.x + v.y, DFT_T1 * v.y - v.x);
 }
 template <bool INV>
 __device__ __forceinline__ float2 lift202(float2 v) {   // a half turn and 22.5
-  return INV ? make_float2(DFT_T1 * v.y - v.x, -DFT_T1 * v.x - v.y)
-             : make_float2(-DFT_T1 * v.y - v.x, DFT_T1 * v.x - v.y);
+  return INV ? make_float2(v.y - DFT_T1 * v.x, -DFT_T1 * v.y - v.x)
+             : make_float2(-DFT_T1 * v.x - v.y, v.x - DFT_T1 * v.y);
 }
 template <bool INV>
 __device__ __forceinline__ float2 lift67(float2 v) {
-  return INV ? make_float2(DFT_T1 * v.x - v.y, v.x + DFT_T1 * v.y)
-             : make_float2(v.y + DFT_T1 * v.x, DFT_T1 * v.y - v.x);
+  return INV ? make_float2(v.x - DFT_T1 * v.y, DFT_T1 * v.x + v.y)
+             : make_float2(DFT_T1 * v.y + v.x, v.y - DFT_T1 * v.x);
 }
 template <bool INV>
 __device__ __forceinline__ float2 lift45(float2 v) {
@@ -180,7 +186,7 @@ __device__ __forceinline__ void dft16_tail(float2 (&v)[16]) {
     v[5] = lift22<INV>(v[5]);
     v[7] = lift67<INV>(v[7]);
     const float2 w = lift45<INV>(v[6]);
-    dft4_scaled<INV>(DFT_C1, cfma(DFT_R2, w, v[4]), cfma(-DFT_R2, w, v[4]), v[4], v[5], v[6], v[7]);
+    dft4_scaled<INV>(DFT_S1, cfma(DFT_R2, w, v[4]), cfma(-DFT_R2, w, v[4]), v[4], v[5], v[6], v[7]);
   }
   {   // k1 = 2: 45, 90, 135
     v[9] = lift45<INV>(v[9]);
@@ -191,7 +197,7 @@ __device__ __forceinline__ void dft16_tail(float2 (&v)[16]) {
     v[13] = lift67<INV>(v[13]);
     const float2 w = lift135<INV>(v[14]);
     v[15] = lift202<INV>(v[15]);
-    dft4_scaled<INV>(DFT_C1, cfma(DFT_R2, w, v[12]), cfma(-DFT_R2, w, v[12]), v[12], v[13], v[14], v[15]);
+    dft4_scaled<INV>(DFT_S1, cfma(DFT_R2, w, v[12]), cfma(-DFT_R2, w, v[12]), v[12], v[13], v[14], v[15]);
   }
 }
 template <bool INV>
