@@ -10,12 +10,14 @@
 //
 // Exactness: blocked, d_eff, oad, f_soften and f_horn reproduce the
 // reference's rounding bit for bit (float32 with float64 where Numba
-// promotes, no FMA contraction).  Blocking samples are classified with a
-// float32 projection first; a sample whose block cell is ambiguous within
-// the float32 error bound (SAMPLE_DELTA cells) is recomputed with the exact
-// float64 mirror, so GB300's low float64 rate is only paid at field edges.
-// Fluence and TERMA run in float32 (reference: float64 fluence, float32
-// TERMA) and are compared with a tolerance.
+// promotes, no FMA contraction) where a call returns them; a dose-only call
+// takes the off-axis distance from pairs of float32 (project_pairs) and adds a
+// map's samples in pairs.  Blocking samples are classified with a float32
+// projection first; a sample whose block cell is ambiguous within the voxel's
+// error bound (lattice_centre; a fixed SAMPLE_DELTA on the general path) is
+// recomputed with the exact float64 mirror, so GB300's low float64 rate is only
+// paid at field edges.  Fluence and TERMA run in float32 (reference: float64
+// fluence, float32 TERMA) and are compared with a tolerance.
 
 #include <algorithm>
 #include <cstdio>
@@ -190,9 +192,9 @@ __device__ __noinline__ float sample_exact(const BeamDev& b, const GridDev& g, c
 }
 
 // ------------------------------------------------------------ blocking --
-// Transmission of sub-sample (ix, iy, iz) at pos + (rx, ry, rz): float32
-// projection, exact float64 mirror only when the block cell is ambiguous
-// within SAMPLE_DELTA.
+// Transmission of sub-sample (ix, iy, iz) at pos + (rx, ry, rz) on the general
+// path: float32 projection, exact float64 mirror only when the block cell is
+// ambiguous within SAMPLE_DELTA.
 __device__ __forceinline__ float sample_value(const BeamDev& b, const GridDev& g, const float* pos,
                                               const float* off, float rx, float ry, float rz, int ix, int iy,
                                               int iz, int& bad) {
@@ -308,6 +310,8 @@ __device__ __forceinline__ bool lattice_centre(const BeamDev& b, const float* po
   return !b.wraps || (c.u - c.mu > -1999.0f && c.w - c.mw > -1999.0f);
 }
 
+// Takes its own look at the voxel: the general path is rare, and a bound handed
+// to it cost 64 mixed beams 1% (registers of every voxel).
 __device__ __noinline__ bool general_exact(const BeamDev& b, const float* pos) {
   Centre c;
   c.delta = 1.0e30f;
@@ -1378,8 +1382,8 @@ void launch_prologue(const float* rho, const GridDev& g, const BeamDev& b, const
 }
 
 // Batched prologue (no intermediates): one cull launch over every beam's grid
-// and one TERMA launch in which each beam's list is shared by the same number
-// of CTAs, so all beams run together and no beam leaves a tail.
+// and one TERMA launch whose warps claim chunks of every beam's list from one
+// counter, so all beams run together and no beam leaves a tail.
 void launch_prologue_batch(const PrologueBeam* recs, int n_beams, long long max_voxels, long long max_lines,
                            int n_sm, int* flags, int* work, cudaStream_t st, int ctas_per_sm) {
   const int threads = 256;

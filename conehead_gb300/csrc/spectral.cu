@@ -480,7 +480,7 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 // first stores), separate the phases (release/acquire) and end it (the
 // partner has read this CTA's half before it exits); every thread reaches
 // each of them once.  Consecutive clusters take the same kz of consecutive
-// pairs, so that plane of S^ comes from L2 after the first.
+// beams, so that plane of S^ comes from L2 after the first.
 constexpr int PLANE_THREADS = 512;
 constexpr int PLANE_WARPS = PLANE_THREADS / 32;
 static_assert(SPEC_PLANE_SMEM >= (128 * 128 + PLANE_WARPS * 2 * 256 + 16 * PLANE_TW_ROW) * 8,
@@ -715,16 +715,15 @@ int spec_length_z(int nz) { return at_least(nz); }
 // quarter steps exp(-2 pi i k / (4 M)), k < 4 M.
 std::vector<float2> spec_twiddles() {
   std::vector<float2> t;
-  auto add = [&](int M, int N) {
+  auto add = [&](int N) {
     for (int k = 0; k < N; ++k) {
       const double a = -2.0 * 3.14159265358979323846 * (double)k / (double)N;
       t.push_back(make_float2((float)std::cos(a), (float)std::sin(a)));
     }
-    (void)M;
   };
   for (int M : spec_lengths()) {
-    add(M, M);
-    add(M, 4 * M);
+    add(M);
+    add(4 * M);
   }
   return t;
 }
