@@ -1386,7 +1386,7 @@ ch_status run_group(ch_plan* P, int n, const ch_grid* grids, const float* const*
   P->last_stream = s;
   if (P->new_call) {          // (a refused call leaves the failures of the one before it to be read)
     P->new_call = false;
-    P->epoch += 1;
+    P->epoch = P->epoch == INT_MAX ? 1 : P->epoch + 1;   // never 0, which reset counters hold
     P->flag_words = 0;
   }
   if (B.spectral && !scatter && !inter && fused_prologue(B)) {
